@@ -22,15 +22,17 @@ FAST = os.environ.get("ST_FASTMATH", "1") == "1"
 MINB_FP32 = os.environ.get("ST_MINB_FP32", "7")
 MINB_FP32G = os.environ.get("ST_MINB_FP32G", "4")
 MINB_FP64 = os.environ.get("ST_MINB_FP64", "1")
+MINB_PAIRS = os.environ.get("ST_MINB_PAIRS", "12")
 UNIT_FLAGS = {
     "st_trace_fp32.cu": (["--use_fast_math"] if FAST else []) + [f"-DST_MINB={MINB_FP32}"],
     "st_trace_fp32_guarded.cu": (["--use_fast_math"] if FAST else []) + [f"-DST_MINB={MINB_FP32G}"],
     "st_trace_fp64.cu": [f"-DST_MINB={MINB_FP64}"],
+    "st_trace_pairs.cu": [f"-DST_PAIR_MINB={MINB_PAIRS}"],
     # the fluid solver rounds every float operation as written (no contraction)
     "st_fluid.cu": ["-fmad=false"],
 }
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
-SOURCES = ["st_trace_fp64.cu", "st_trace_fp32.cu", "st_trace_fp32_guarded.cu", "st_api.cu", "st_surrogate.cu", "st_noalloc.cu",
+SOURCES = ["st_trace_fp64.cu", "st_trace_pairs.cu", "st_trace_fp32.cu", "st_trace_fp32_guarded.cu", "st_api.cu", "st_surrogate.cu", "st_noalloc.cu",
            "st_layered.cu", "st_rawio.cpp", "st_fluid.cu", "st_peak.cu"]
 
 

@@ -756,6 +756,7 @@ int do_render(st_context* ctx, const st_camera* cam, const st_spacetime* stp, co
   if ((rc = ensure(&ctx->d_fb, &ctx->fb_cap, npix)) != ST_OK) return rc;
   if (host_rgb && (rc = ensure(&ctx->d_rgb, &ctx->rgb_cap, 3 * npix)) != ST_OK) return rc;
   if (host_diag && (rc = ensure(&ctx->d_diag, &ctx->diag_cap, npix)) != ST_OK) return rc;
+  p.r_max = p.r_escape;
   p.out = ctx->d_fb;
   p.diag = host_diag ? ctx->d_diag : nullptr;
   p.ap_r = cam->aperture_world > 0.0 ? cam->aperture_world / 2.0 : 0.0;
@@ -1636,6 +1637,7 @@ int st_render_frames(st_context* ctx, int nframes, const st_camera* cams, const 
     fc[f].nmax = q.nmax;
     fc[f].pad = 0;
     nmax_max = std::max(nmax_max, q.nmax);
+    p.r_max = std::max(p.r_max, q.r_escape);
   }
   if ((rc = ensure(&ctx->d_frames, &ctx->frames_cap, (size_t)nframes)) != ST_OK) return rc;
   if ((rc = ensure(&ctx->d_fb, &ctx->fb_cap, npix * nframes)) != ST_OK) return rc;

@@ -5,7 +5,10 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <cmath>
+
 #include "../../include/spacetime_gb300.h"
+#include "st_df.cuh"
 
 namespace st {
 
@@ -162,7 +165,15 @@ struct TraceParams {
     // gas emission: 1 / (2M), 100 emis, opac ds_gas log2(e)
     float inv_2m, emis100, opds_l2;
   } f;
+  // the same as float pairs, for the FP64 frames that integrate on the FP32 pipe
+  dfm::Scene d;
+  double r_max;              // largest escape radius of the launch's frames (0: not known)
 };
+
+inline df2 host_pair(double v) {
+  const float h = (float)v;
+  return df2{h, (float)(v - (double)h)};
+}
 
 // Fill TraceParams::f from the double fields (host, after they are set).
 inline void fill_float_copies(TraceParams* p) {
@@ -211,6 +222,33 @@ inline void fill_float_copies(TraceParams* p) {
   p->f.inv_2m = (float)(1.0 / (2.0 * p->M));
   p->f.emis100 = (float)(100.0 * p->emis);
   p->f.opds_l2 = (float)(p->opac * p->ds_gas * 1.4426950408889634);
+  dfm::Scene& d = p->d;
+  d.H = dfm::Hole{host_pair(p->M), host_pair(p->a), host_pair(p->a * p->a)};
+  d.dt = host_pair(p->dt);
+  d.hcoef = host_pair(p->hcoef / p->M);
+  d.inv_rkill2 = host_pair(1.0 / rkd);
+  d.r32 = host_pair(3.2 * p->M);
+  d.r295 = host_pair(2.95 * p->M);
+  d.ds = host_pair(p->ds_gas);
+  d.ds_span = host_pair(p->opac * p->ds_gas);
+  d.ln_in = host_pair(p->ls_in);
+  d.ln_out = host_pair(p->ls_out);
+  d.kr = host_pair(sr);
+  d.kphi = host_pair(p->nphi / 6.283185307179586);
+  d.kz = host_pair(p->zmax > 0.0 ? (p->nz - 1) / (2.0 * p->zmax) : 0.0);
+  d.klut = host_pair(p->lut_tmax > p->lut_tmin ? (p->lut_size - 1) / (p->lut_tmax - p->lut_tmin) : 0.0);
+  d.tmin = host_pair(p->lut_tmin);
+  d.tmax = host_pair(p->lut_tmax);
+  d.emis100 = host_pair(100.0 * p->emis);
+  d.T0 = host_pair(std::exp(10.034259));
+  d.isco = host_pair(p->r_isco);
+  d.inv_isco = host_pair(1.0 / p->r_isco);
+  d.E = host_pair(p->E_isco);
+  d.L = host_pair(p->L_isco);
+  d.sqM = host_pair(std::sqrt(p->M));
+  d.inv_2m = host_pair(1.0 / (2.0 * p->M));
+  d.rb2 = host_pair(p->vol_rb2);
+  d.tspan = host_pair(p->tspan);
 }
 
 // Variant key of the compiled kernels (the reference's Val{...} switches,

@@ -1185,9 +1185,6 @@ __device__ __forceinline__ void guard_step_fp64(float* y, float* lo, float pt, d
 // operation is a rounded intrinsic, so neither contraction nor fast-math
 // flags of the translation unit change the error-free transformations.
 // ---------------------------------------------------------------------------
-struct df2 {
-  float hi, lo;
-};
 __device__ __forceinline__ df2 dfq(float a) { return df2{a, 0.f}; }
 __device__ __forceinline__ df2 df_two_sum(float a, float b) {
   const float s = __fadd_rn(a, b);
