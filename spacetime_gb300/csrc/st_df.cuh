@@ -279,6 +279,30 @@ ST_DF t3 add3(t3 y, dd c) {
   return t3{v2_.h, w2.h, w2.l};
 }
 
+// to and from double
+ST_DF df2 pair_of(double v) {
+  const float h = (float)v;
+  return df2{h, (float)(v - (double)h)};
+}
+ST_DF f3 f3_of(double v) {
+  const float h = (float)v;
+  const double r = v - (double)h;
+  const float m = (float)r;
+  return f3{h, m, (float)(r - (double)m)};
+}
+ST_DF double dbl(df2 x) { return (double)x.hi + (double)x.lo; }
+ST_DF double dbl(f3 x) { return (double)x.h + ((double)x.m + (double)x.l); }
+// (x, y, z, p_x, p_y, p_z) of a ray's state, and back
+ST_DF void doubles(const t3& P, const t3& Q, const t3& W, double* y) {
+  y[0] = dbl(fst(P)); y[1] = dbl(snd(P)); y[2] = dbl(fst(W));
+  y[3] = dbl(fst(Q)); y[4] = dbl(snd(Q)); y[5] = dbl(snd(W));
+}
+ST_DF void set_state(const double* y, t3* P, t3* Q, t3* W) {
+  *P = two(f3_of(y[0]), f3_of(y[1]));
+  *Q = two(f3_of(y[3]), f3_of(y[4]));
+  *W = two(f3_of(y[2]), f3_of(y[5]));
+}
+
 // ---------------------------------------------------------------------------
 // Geodesic right-hand sides (the regrouped forms of st_trace.cuh).
 // ---------------------------------------------------------------------------
@@ -383,6 +407,40 @@ ST_DF void rhs(dd P, dd Q, dd W, const Geo& g, df2 pt, const Hole& H, dd* dP, dd
     *dQ = dot2(C1, Q, n2, P);
     *dW = two(fma1(neg(c1), z, pz), dot2(c1, pz, neg(c2), z));
   }
+}
+
+// Classical RK4: the increments of one step of size *h from (P, Q, W).  begin(g, h)
+// sees the geometry of the state, sets the step's size and may end the ray;
+// first(dP, dW) sees the slopes at the state.  The four stages share one copy
+// of the right-hand side.
+template <int KERR, class Begin, class First>
+ST_DF bool rk4(const t3& P, const t3& Q, const t3& W, df2 pt, const Hole& H, const Begin& begin, const First& first,
+               df2* h, dd* iP, dd* iQ, dd* iW) {
+  dd tP = top(P), tQ = top(Q), tW = top(W);
+  dd sP = two(q(0.f), q(0.f)), sQ = sP, sW = sP;
+#ifdef __CUDACC__
+#pragma unroll 1
+#endif
+  for (int s = 0; s < 4; ++s) {
+    const Geo g = geometry<KERR>(tP, fst(tW), H);
+    if (s == 0 && begin(g, h)) return true;
+    dd kP, kQ, kW;
+    rhs<KERR>(tP, tQ, tW, g, pt, H, &kP, &kQ, &kW);
+    if (s == 0) first(kP, kW);
+    const float w = (s == 1 || s == 2) ? 2.f : 1.f;
+    sP = add(sP, scale(kP, w));
+    sQ = add(sQ, scale(kQ, w));
+    sW = add(sW, scale(kW, w));
+    const dd hs = both(scale(*h, s < 2 ? 0.5f : 1.f));
+    tP = fma1(hs, kP, top(P));
+    tQ = fma1(hs, kQ, top(Q));
+    tW = fma1(hs, kW, top(W));
+  }
+  const dd h6 = both(mul(*h, df2{0.166666672f, -4.96705388e-9f}));
+  *iP = mul(h6, sP);
+  *iQ = mul(h6, sQ);
+  *iW = mul(h6, sW);
+  return false;
 }
 
 // ---------------------------------------------------------------------------

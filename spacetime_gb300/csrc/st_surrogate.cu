@@ -22,7 +22,7 @@
 // accumulation (st_mlp.cuh); the 6->256 and 256->6 layers, the loss and AdamW
 // run in FP32.  Master weights and optimiser state are FP32.
 //
-// Training labels come from the FP64 integrator on the GPU (label_kernel):
+// Training labels come from the FP64 integrator on the GPU (label_pairs_kernel):
 // Sobol-sampled inputs, the kernel's step rule and kill tests
 // (src/metal.jl:1201-1572) with the spin per sample, exit direction on the
 // escape radius 2 max(|pos|, 15M) (src/metal.jl:2058-2059).
@@ -443,6 +443,9 @@ struct LabelParams {
   float* raw;         // optional [n][15]: r, theta, a, n0, n1, n2, flags, steps, exit dir (3), r_cross,
                       // launch coordinate direction d0 (3)
   double dt;
+  // the last `sorted` samples are taken in this order (label_order): rows
+  const uint32_t* order;
+  long long sorted;
 };
 
 __device__ __forceinline__ void normalise_inputs(float r, float th, float a, const float* n, float* x) {
@@ -454,63 +457,375 @@ __device__ __forceinline__ void normalise_inputs(float r, float th, float a, con
   x[5] = n[2];
 }
 
-// FP64 integration of one sample with the kernel's rules (no gas, no disc
-// shading): exit direction on r_escape (landed), first z = 0 crossing radius
-// and 1/(1+z) of the exact emitter there.
-__global__ void label_kernel(const LabelParams lp) {
-  const long long tid = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (tid >= lp.n) return;
-  const uint32_t idx = (uint32_t)(lp.offset + tid + 1);  // skip the origin point
-  const float u0 = sobol(idx, 0), u1 = sobol(idx, 1), u2 = sobol(idx, 2), u3 = sobol(idx, 3), u4 = sobol(idx, 4);
-  const double r = 4.0 + 46.0 * u0;
-  const double th = 1.5707963267948966 * u1;
-  const double a = 0.99 * u2;
+// r and the cosine to the inward radial direction of a sample.
+__device__ __forceinline__ double label_cosine(float u3) {
   // directions: 80% uniform on the 75-degree cone around the inward radial
   // axis (every camera that looks at the hole sees its whole frame inside it),
   // 20% uniform on the rest of the sphere
   const double cmin = 0.25881904510252074;  // cos 75 deg
-  const double ca = (u3 < 0.8f) ? 1.0 - (double)(u3 / 0.8f) * (1.0 - cmin)
-                                : cmin - (double)((u3 - 0.8f) / 0.2f) * (1.0 + cmin);
+  return (u3 < 0.8f) ? 1.0 - (double)(u3 / 0.8f) * (1.0 - cmin)
+                     : cmin - (double)((u3 - 0.8f) / 0.2f) * (1.0 + cmin);
+}
+
+// The steps a sample's ray will take, roughly (correlation 0.95 with the counted
+// ones), in one of ORDER_BUCKETS classes, longest first: the straight line at
+// its impact parameter b, walked at the step rule h = dt max(0.16 r, 1) out to
+// twice the larger of r and 15 M or into the hole, the bending (which adds
+// about 1250 / (b - 2.5) steps), and 900 steps for a ray that the launch test
+// finds near the critical curve.
+constexpr int ORDER_BUCKETS = 64;
+constexpr long long ORDER_MAX = 1 << 20;
+__device__ __forceinline__ int label_bucket(uint32_t idx) {
+  const float r = 4.f + 46.f * sobol(idx, 0), th = 1.57079633f * sobol(idx, 1), a = 0.99f * sobol(idx, 2);
+  const float c = (float)label_cosine(sobol(idx, 3)), s = sqrtf(fmaxf(1.f - c * c, 0.f));
+  const float b = r * s * rsqrtf(1.f - 2.f / r), re = 2.f * fmaxf(r, 15.f);
+  const bool falls = c > 0.f && b < 4.8f;
+  const float rp = falls ? 1.5f : fmaxf(b - 1.f, 2.f);
+  const float s0 = sqrtf(fmaxf(6.25f * 6.25f - rp * rp, 0.f)), a0 = asinhf(s0 / rp);
+  auto leg = [&](float r1) {  // periapsis to r1, in units of 50 steps at dt = 0.02
+    const float s1 = sqrtf(fmaxf(r1 * r1 - rp * rp, 0.f));
+    return s1 <= s0 ? s1 : s0 + 6.25f * (asinhf(s1 / rp) - a0);
+  };
+  float n = falls ? leg(r) + 4.f : (c > 0.f ? leg(re) + leg(r) + 25.f / (b - 2.5f) : leg(re) - leg(r));
+  if (c > 0.f && b > 2.f && b < 7.5f) {
+    // the launch test of the double code, in float
+    float sp, cp;
+    sincosf(6.28318531f * sobol(idx, 4), &sp, &cp);
+    const float pos[3] = {sqrtf(r * r + a * a) * sinf(th), 0.f, r * cosf(th)};
+    float e1[3], e2[3], e3[3], U[4], E1[4], E2[4], E3[4], q[4], y[6], pt;
+    frame_axes(pos, e1, e2, e3);
+    static_frame(pos, e1, e2, e3, 1.f, a, U, E1, E2, E3);
+    for (int k = 0; k < 4; ++k) q[k] = -c * E1[k] + s * cp * E2[k] + s * sp * E3[k] - U[k];
+    lower_photon<1>(pos, q, 1.f, a, y, &pt);
+    bool cap = false, graze = false;
+    bardeen(y, pt, 1.f, a, &cap, &graze);
+    if (graze) n += 18.f;
+  }
+  return ORDER_BUCKETS - 1 - min(max((int)(n * (50.f / 2600.f * ORDER_BUCKETS)), 0), ORDER_BUCKETS - 1);
+}
+
+// Counting sort of the rows n - m .. n - 1 by that class: histogram, then places.
+__global__ void __launch_bounds__(256) label_count(long long first, long long offset, int m, unsigned* hist) {
+  __shared__ unsigned h[ORDER_BUCKETS];
+  if (threadIdx.x < ORDER_BUCKETS) h[threadIdx.x] = 0;
+  __syncthreads();
+  const int i = blockIdx.x * 256 + threadIdx.x;
+  if (i < m) atomicAdd(h + label_bucket((uint32_t)(offset + first + i + 1)), 1u);
+  __syncthreads();
+  if (threadIdx.x < ORDER_BUCKETS && h[threadIdx.x]) atomicAdd(hist + threadIdx.x, h[threadIdx.x]);
+}
+__global__ void __launch_bounds__(256) label_place(long long first, long long offset, int m, const unsigned* hist,
+                                                   unsigned* used, uint32_t* order) {
+  __shared__ unsigned h[ORDER_BUCKETS], base[ORDER_BUCKETS];
+  if (threadIdx.x < ORDER_BUCKETS) h[threadIdx.x] = 0;
+  __syncthreads();
+  const int i = blockIdx.x * 256 + threadIdx.x;
+  int b = 0;
+  unsigned k = 0;
+  if (i < m) {
+    b = label_bucket((uint32_t)(offset + first + i + 1));
+    k = atomicAdd(h + b, 1u);
+  }
+  __syncthreads();
+  if (threadIdx.x < ORDER_BUCKETS) {
+    unsigned before = 0;
+    for (int c = 0; c < (int)threadIdx.x; ++c) before += hist[c];
+    base[threadIdx.x] = before + (h[threadIdx.x] ? atomicAdd(used + threadIdx.x, h[threadIdx.x]) : 0u);
+  }
+  __syncthreads();
+  if (i < m) order[base[b] + k] = (uint32_t)(first + i);
+}
+
+// One sample's ray at launch.
+struct LabelRay {
+  double y[6], pt, a, r_esc, rkill2;
+  int nmax;
+  bool cap0, graze0;
+  // what the outputs need besides
+  double r, th, nv[3], pos[3], rpos, d0[3];
+};
+
+// Sample idx of the Sobol sequence: camera, spin and direction, the ray they
+// launch, and the rules of the kernel for it (src/metal.jl:347-357, 1201-1260,
+// 2058-2062).
+__device__ __forceinline__ void label_launch(uint32_t idx, double dt, LabelRay& L) {
+  const float u0 = sobol(idx, 0), u1 = sobol(idx, 1), u2 = sobol(idx, 2), u3 = sobol(idx, 3), u4 = sobol(idx, 4);
+  const double r = 4.0 + 46.0 * u0;
+  const double th = 1.5707963267948966 * u1;
+  const double a = 0.99 * u2;
+  const double ca = label_cosine(u3);
   const double sa = sqrt(fmax(1.0 - ca * ca, 0.0)), ph = 6.283185307179586 * u4;
-  const double nv[3] = {-ca, sa * cos(ph), sa * sin(ph)};
+  L.nv[0] = -ca; L.nv[1] = sa * cos(ph); L.nv[2] = sa * sin(ph);
+  L.r = r; L.th = th; L.a = a;
   const double M = 1.0;
-  const double pos[3] = {sqrt(r * r + a * a) * sin(th), 0.0, r * cos(th)};
+  L.pos[0] = sqrt(r * r + a * a) * sin(th); L.pos[1] = 0.0; L.pos[2] = r * cos(th);
   double e1[3], e2[3], e3[3], U[4], E1[4], E2[4], E3[4];
-  frame_axes(pos, e1, e2, e3);
-  static_frame(pos, e1, e2, e3, M, a, U, E1, E2, E3);
+  frame_axes(L.pos, e1, e2, e3);
+  static_frame(L.pos, e1, e2, e3, M, a, U, E1, E2, E3);
   double q[4];
-  for (int k = 0; k < 4; ++k) q[k] = nv[0] * E1[k] + nv[1] * E2[k] + nv[2] * E3[k] - U[k];
-  double y[6], pt;
-  if (a != 0.0) lower_photon<1>(pos, q, M, a, y, &pt);
-  else lower_photon<0>(pos, q, M, a, y, &pt);
-  bool cap0 = false, graze0 = false;
-  if (a != 0.0) bardeen(y, pt, M, a, &cap0, &graze0);
+  for (int k = 0; k < 4; ++k) q[k] = L.nv[0] * E1[k] + L.nv[1] * E2[k] + L.nv[2] * E3[k] - U[k];
+  if (a != 0.0) lower_photon<1>(L.pos, q, M, a, L.y, &L.pt);
+  else lower_photon<0>(L.pos, q, M, a, L.y, &L.pt);
+  L.cap0 = L.graze0 = false;
+  if (a != 0.0) bardeen(L.y, L.pt, M, a, &L.cap0, &L.graze0);
   // initial coordinate direction (the residual's base)
   double k1[6];
-  rhs_kerr(y, pt, M, a, k1);
+  rhs_kerr(L.y, L.pt, M, a, k1);
   const double v0n = sqrt(k1[0] * k1[0] + k1[1] * k1[1] + k1[2] * k1[2]);
-  const double d0[3] = {k1[0] / v0n, k1[1] / v0n, k1[2] / v0n};
-  // rules of the kernel (src/metal.jl:347-357, 1201-1260, 2058-2062)
+  for (int k = 0; k < 3; ++k) L.d0[k] = k1[k] / v0n;
   const double rph = (a == 0.0) ? 3.0 * M : 2.0 * M * (1.0 + cos((2.0 / 3.0) * acos(-a / M)));
   const float rkf = (float)(0.995 * rph);
-  const double rkill2 = (double)(rkf * rkf);
-  const double rpos = sqrt(pos[0] * pos[0] + pos[1] * pos[1] + pos[2] * pos[2]);
-  const double r_esc = (double)(float)(2.0 * fmax(rpos, 15.0 * M));
-  const int nmax = (int)fmin(fmax(1000.0, ceil((75.0 + 6.5 * log(r_esc / M)) * M / lp.dt)), 40000.0);
-  double r_isco, E_isco, L_isco;
-  {
+  L.rkill2 = (double)(rkf * rkf);
+  L.rpos = sqrt(L.pos[0] * L.pos[0] + L.pos[1] * L.pos[1] + L.pos[2] * L.pos[2]);
+  L.r_esc = (double)(float)(2.0 * fmax(L.rpos, 15.0 * M));
+  L.nmax = (int)fmin(fmax(1000.0, ceil((75.0 + 6.5 * log(L.r_esc / M)) * M / dt)), 40000.0);
+}
+
+// The outputs of a sample: its launch, end state y and flags, and the state
+// (x, y, p_x, p_y) c of its first z = 0 crossing (crossed).
+__device__ __forceinline__ void label_write(const LabelParams& lp, long long tid, const LabelRay& L, const double* y,
+                                            int flags, int steps, bool crossed, const double* c) {
+  const double M = 1.0, a = L.a;
+  float r_cross = -1.f, g_cross = 0.f;
+  if (crossed) {
     auto cb = [](double x) { return exp(log(fmax(x, 1e-12)) / 3.0); };
     const double qq = a / M;
     const double z1 = 1.0 + cb(1.0 - qq * qq) * (cb(1.0 + qq) + cb(1.0 - qq));
     const double z2 = sqrt(3.0 * qq * qq + z1 * z1);
-    r_isco = M * (3.0 + z2 - sqrt(fmax((3.0 - z1) * (3.0 + z1 + 2.0 * z2), 0.0)));
-    E_isco = sqrt(1.0 - 2.0 * M / (3.0 * r_isco));
-    L_isco = (2.0 * M / (3.0 * sqrt(3.0))) * (1.0 + 2.0 * sqrt(3.0 * r_isco / M - 2.0));
+    const double r_isco = M * (3.0 + z2 - sqrt(fmax((3.0 - z1) * (3.0 + z1 + 2.0 * z2), 0.0)));
+    const double E_isco = sqrt(1.0 - 2.0 * M / (3.0 * r_isco));
+    const double L_isco = (2.0 * M / (3.0 * sqrt(3.0))) * (1.0 + 2.0 * sqrt(3.0 * r_isco / M - 2.0));
+    r_cross = (float)sqrt(c[0] * c[0] + c[1] * c[1]);
+    g_cross = (float)(1.0 / emitter_opz(c[0], c[1], c[2], c[3], -L.pt, M, a, r_isco, E_isco, L_isco));
   }
+  if (!(flags & (ST_RAY_ESCAPED | ST_RAY_CAPTURED))) flags |= ST_RAY_BUDGET;
+  if (L.cap0) flags |= ST_RAY_BCAPT;
+  if (L.graze0) flags |= ST_RAY_GRAZE;
+  double vel[6];
+  rhs_kerr(y, L.pt, M, a, vel);
+  const double vl = fmax(sqrt(vel[0] * vel[0] + vel[1] * vel[1] + vel[2] * vel[2]), 1e-20);
+  const bool ok = (flags & ST_RAY_ESCAPED) && !L.cap0 && !(flags & ST_RAY_BUDGET);
+  float x[6];
+  const float nf[3] = {(float)L.nv[0], (float)L.nv[1], (float)L.nv[2]};
+  normalise_inputs((float)L.r, (float)L.th, (float)a, nf, x);
+  float* Xo = lp.X + tid * NIN;
+  for (int k = 0; k < NIN; ++k) Xo[k] = x[k];
+  float* To = lp.T + tid * NT;
+  double defl = 0.0, tilt = 0.0;
+  if (ok) {
+    const double xh[3] = {L.pos[0] / L.rpos, L.pos[1] / L.rpos, L.pos[2] / L.rpos};
+    const double dex[3] = {vel[0] / vl, vel[1] / vl, vel[2] / vl};
+    plane_angles(xh, L.d0, dex, &defl, &tilt);
+  }
+  To[0] = (float)defl;
+  To[1] = (float)tilt;
+  To[2] = 0.f;
+  To[3] = (r_cross > 0.f ? fminf(10.f / r_cross, 5.f) : 0.f) - 1.f;  // 10/s - 1; no crossing = s -> inf
+  To[4] = r_cross > 0.f ? g_cross - 1.f : 0.f;
+  To[5] = ok ? 1.f : 0.f;
+  To[6] = r_cross > 0.f ? 1.f : 0.f;
+  To[7] = 0.f;
+  if (lp.raw) {
+    float* Ro = lp.raw + tid * NRAW;
+    Ro[0] = (float)L.r; Ro[1] = (float)L.th; Ro[2] = (float)a;
+    Ro[3] = nf[0]; Ro[4] = nf[1]; Ro[5] = nf[2];
+    Ro[6] = (float)flags; Ro[7] = (float)steps;
+    Ro[8] = (float)(vel[0] / vl); Ro[9] = (float)(vel[1] / vl); Ro[10] = (float)(vel[2] / vl);
+    Ro[11] = r_cross;
+    Ro[12] = (float)L.d0[0]; Ro[13] = (float)L.d0[1]; Ro[14] = (float)L.d0[2];
+  }
+}
+
+// FP64 labels: each sample's ray integrated with the kernel's rules (no gas, no
+// disc shading), its exit direction on r_escape (landed), its first z = 0
+// crossing radius and 1/(1+z) of the exact emitter there.
+//
+// The integration runs in float pairs (dfm::rk4, as the FP64 frames).  Sobol
+// neighbours share nothing, so with one ray a thread a warp waited for its
+// longest ray with 14 of 32 lanes busy.  Here a warp is its own queue: a lane
+// whose ray ends leaves it in the warp's list of ended rays and takes the next
+// launched one.  Launch and outputs are double code (its cost is per warp, not
+// per lane), so they run 32 at a time: launches when the list of launched rays
+// is empty, outputs when that of ended ones is full.  The last million samples
+// are taken longest first (label_order), so the warps drain on short rays.
+// 131,072 labels: 302 ms all in double with one ray a thread, 31 ms so, 27 ms in
+// order, 24 ms with fewer warps; at 2^20 it is 8.3 M labels a second (0.44 M).
+// Bound by the FP32 pipe (70 %), small sets by their longest ray.
+struct LabelWarp {
+  // launched rays, to be taken from `next` on
+  dfm::t3 P[32], Q[32], W[32];
+  df2 pt[32], a[32], a2[32];
+  float rkill2[32], r_esc[32];
+  int nmax[32];
+  // ended rays
+  dfm::t3 eP[32], eQ[32], eW[32];
+  df2 eh[32], c[4][32];
+  int eflags[32], esteps[32];
+  uint32_t row[32], erow[32];
+};
+constexpr int LABEL_WARPS = 8;  // per SM
+__global__ void __launch_bounds__(32, LABEL_WARPS) label_pairs_kernel(const LabelParams lp, unsigned* queue) {
+  using namespace dfm;
+  __shared__ LabelWarp g;
+  const unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x;
+  const unsigned below = (1u << lane) - 1u;
+  const df2 dt = pair_of(lp.dt);
+  t3 P, Q, W;
+  df2 pt, land{0.f, 0.f}, c0{-1.f, 0.f}, c1{0.f, 0.f}, c2{0.f, 0.f}, c3{0.f, 0.f};
+  Hole H;
+  H.M = q(1.f);
+  float rkill2 = 0.f, r_esc = 0.f;
+  int nmax = 0, steps = 0, flags = 0;
+  uint32_t row = 0;
+  bool run = false, crossed = false;
+  int next = 0, have = 0, ended = 0;  // uniform over the warp
+  bool drained = false;
+  for (;;) {
+    unsigned idle = __ballot_sync(FULL, !run);
+    while (idle && !(drained && next == have)) {
+      if (next == have) {
+        unsigned base = 0;
+        if (lane == 0) base = atomicAdd(queue, 32u);
+        base = __shfl_sync(FULL, base, 0);
+        next = 0;
+        have = (long long)base < lp.n ? (int)min(32ll, lp.n - (long long)base) : 0;
+        if (have == 0) { drained = true; break; }
+        if (lane < have) {
+          const long long k = (long long)base + lane, plain = lp.n - lp.sorted;
+          const uint32_t rr = k < plain ? (uint32_t)k : lp.order[k - plain];
+          LabelRay L;
+          label_launch((uint32_t)(lp.offset + rr + 1), lp.dt, L);  // skip the origin point
+          set_state(L.y, &g.P[lane], &g.Q[lane], &g.W[lane]);
+          g.pt[lane] = pair_of(L.pt);
+          g.a[lane] = pair_of(L.a);
+          g.a2[lane] = pair_of(L.a * L.a);
+          g.rkill2[lane] = (float)L.rkill2;
+          g.r_esc[lane] = (float)L.r_esc;
+          g.nmax[lane] = L.nmax;
+          g.row[lane] = rr;
+        }
+        __syncwarp();
+      }
+      const int k = next + __popc(idle & below);
+      if (!run && k < have) {
+        P = g.P[k]; Q = g.Q[k]; W = g.W[k];
+        pt = g.pt[k]; H.a = g.a[k]; H.a2 = g.a2[k];
+        rkill2 = g.rkill2[k]; r_esc = g.r_esc[k]; nmax = g.nmax[k]; row = g.row[k];
+        land = q(0.f);
+        steps = flags = 0;
+        crossed = false;
+        run = true;
+      }
+      __syncwarp();
+      next = min(have, next + __popc(idle));
+      idle = __ballot_sync(FULL, !run);
+    }
+    const bool last = !__any_sync(FULL, run);  // no ray left: write out the rest
+    bool end = false;
+    if (run) {
+      df2 h;
+      dd iP, iQ, iW;
+      end = steps >= nmax;
+      if (!end)
+        end = rk4<1>(
+            P, Q, W, pt, H,
+            [&](const Geo& g1, df2* hh) {
+              if (lt(g1.r2, q(rkill2))) { flags |= ST_RAY_CAPTURED; return true; }
+              const df2 r = sqrt_(g1.flat2);
+              if (lt(q(r_esc), r)) { flags |= ST_RAY_ESCAPED; return true; }
+              const df2 hb = min_(max_(mul(df2{0.159999996f, 3.57627866e-9f}, r), q(1.f)), q(8.f));  // 0.16 r
+              const df2 ik = rcp(max_(q(rkill2), df2{9.99999997e-7f, 2.52435490e-15f}));
+              const df2 fr = min_(max_(mul(addf(g1.r2, -rkill2), ik), q(0.f)), q(1.f));
+              *hh = mul(mul(dt, hb), fma1(df2{0.879999995f, 4.76837159e-9f}, fr, df2{0.119999997f, 2.68220901e-9f}));
+              return false;
+            },
+            [](const dd&, const dd&) {}, &h, &iP, &iQ, &iW);
+      if (!end) {
+        const t3 P0 = P, Q0 = Q, W0 = W;
+        P = add3(P, iP);
+        Q = add3(Q, iQ);
+        W = add3(W, iW);
+        const float z0 = W0.h.x, z1 = W.h.x;
+        if (!(P.h.x == P.h.x) || !(Q.h.x == Q.h.x)) {
+          flags |= ST_RAY_CAPTURED;
+          end = true;
+        } else {
+          ++steps;
+          if (!crossed && ((z0 < 0.f && z1 > 0.f) || (z0 > 0.f && z1 < 0.f))) {
+            // the state where z = 0, linear in the step
+            const df2 f = mul(fst(top(W0)), rcp(neg(fst(iW))));
+            const dd p = fma1(both(f), iP, top(P0)), m = fma1(both(f), iQ, top(Q0));
+            c0 = fst(p); c1 = snd(p); c2 = fst(m); c3 = snd(m);
+            crossed = true;
+          }
+          const float r2f = fmaf(P.h.x, P.h.x, fmaf(P.h.y, P.h.y, z1 * z1));
+          if (r2f > 0.9999f * r_esc * r_esc) {
+            const df2 r2n = sumsq(fst(top(P)), snd(top(P)), fst(top(W)), q(0.f));
+            if (lt(mul(q(r_esc), q(r_esc)), r2n)) {
+              // landed on r_escape, as the render path does, when the outputs are written
+              P = P0; Q = Q0; W = W0;
+              land = h;
+              flags |= ST_RAY_ESCAPED;
+              end = true;
+            }
+          }
+        }
+      }
+      if (end) run = false;
+    }
+    const unsigned fin = __ballot_sync(FULL, end);
+    // outputs of the ended rays: when this step's no longer fit, and at the end
+#pragma unroll 1
+    for (int round = 0; round < 2; ++round) {
+      const int n = __popc(fin);
+      if (round == 0 ? ended + n > 32 : last && ended > 0) {
+        if (lane < ended) {
+          LabelRay L;
+          const uint32_t rr = g.erow[lane];
+          label_launch((uint32_t)(lp.offset + rr + 1), lp.dt, L);
+          double y[6];
+          doubles(g.eP[lane], g.eQ[lane], g.eW[lane], y);
+          if (g.eh[lane].hi > 0.f) land_in_step<1>(y, L.pt, 1.0, L.a, dbl(g.eh[lane]), L.r_esc);
+          double c[4];
+          for (int k = 0; k < 4; ++k) c[k] = dbl(g.c[k][lane]);
+          const int fl = g.eflags[lane];
+          label_write(lp, (long long)rr, L, y, fl & ~ST_RAY_CROSSED, g.esteps[lane], (fl & ST_RAY_CROSSED) != 0, c);
+        }
+        __syncwarp();
+        ended = 0;
+      }
+      if (round == 0 && n > 0) {
+        if (end) {
+          const int k = ended + __popc(fin & below);
+          g.eP[k] = P; g.eQ[k] = Q; g.eW[k] = W;
+          g.eh[k] = land;
+          g.c[0][k] = c0; g.c[1][k] = c1; g.c[2][k] = c2; g.c[3][k] = c3;
+          g.eflags[k] = flags | (crossed ? ST_RAY_CROSSED : 0);
+          g.esteps[k] = steps;
+          g.erow[k] = row;
+        }
+        __syncwarp();
+        ended += n;
+      }
+    }
+    if (last) break;
+  }
+}
+
+// The same all in double, one ray a thread: steps outside the pair kernel's
+// range (see pairs_take in st_trace_pairs.cu).
+__global__ void label_kernel(const LabelParams lp) {
+  const long long tid = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (tid >= lp.n) return;
+  LabelRay L;
+  label_launch((uint32_t)(lp.offset + tid + 1), lp.dt, L);  // skip the origin point
+  const double M = 1.0, a = L.a, pt = L.pt, rkill2 = L.rkill2, r_esc = L.r_esc;
+  double y[6], k1[6], c[4] = {0, 0, 0, 0};
+  for (int k = 0; k < 6; ++k) y[k] = L.y[k];
   int flags = 0, steps = 0;
-  float r_cross = -1.f, g_cross = 0.f;
-  bool done = false;
-  for (; steps < nmax && !done; ++steps) {
+  bool crossed = false, done = false;
+  for (; steps < L.nmax && !done; ++steps) {
     const double r2 = y[0] * y[0] + y[1] * y[1] + y[2] * y[2];
     const double rr = sqrt(r2);
     const double rk2 = ks_r2(y[0], y[1], y[2], a);
@@ -525,12 +840,11 @@ __global__ void label_kernel(const LabelParams lp) {
     rk4_inc<1>(y, pt, M, a, h, k1, inc);
     for (int k = 0; k < 6; ++k) y[k] += inc[k];
     if (!(y[0] == y[0]) || !(y[3] == y[3])) { flags |= ST_RAY_CAPTURED; break; }
-    if (r_cross < 0.f && yp[2] * y[2] < 0.0) {
+    if (!crossed && yp[2] * y[2] < 0.0) {
       const double cfz = yp[2] / (yp[2] - y[2]);
-      const double xh = yp[0] + cfz * (y[0] - yp[0]), yh = yp[1] + cfz * (y[1] - yp[1]);
-      const double pxh = yp[3] + cfz * (y[3] - yp[3]), pyh = yp[4] + cfz * (y[4] - yp[4]);
-      r_cross = (float)sqrt(xh * xh + yh * yh);
-      g_cross = (float)(1.0 / emitter_opz(xh, yh, pxh, pyh, -pt, M, a, r_isco, E_isco, L_isco));
+      const int at[4] = {0, 1, 3, 4};
+      for (int k = 0; k < 4; ++k) c[k] = yp[at[k]] + cfz * (y[at[k]] - yp[at[k]]);
+      crossed = true;
     }
     const double rn = sqrt(y[0] * y[0] + y[1] * y[1] + y[2] * y[2]);
     if (rn > r_esc) {
@@ -542,42 +856,7 @@ __global__ void label_kernel(const LabelParams lp) {
       done = true;
     }
   }
-  if (!(flags & (ST_RAY_ESCAPED | ST_RAY_CAPTURED))) flags |= ST_RAY_BUDGET;
-  if (cap0) flags |= ST_RAY_BCAPT;
-  if (graze0) flags |= ST_RAY_GRAZE;
-  double vel[6];
-  rhs_kerr(y, pt, M, a, vel);
-  const double vl = fmax(sqrt(vel[0] * vel[0] + vel[1] * vel[1] + vel[2] * vel[2]), 1e-20);
-  const bool ok = (flags & ST_RAY_ESCAPED) && !cap0 && !(flags & ST_RAY_BUDGET);
-  float x[6];
-  const float nf[3] = {(float)nv[0], (float)nv[1], (float)nv[2]};
-  normalise_inputs((float)r, (float)th, (float)a, nf, x);
-  float* Xo = lp.X + tid * NIN;
-  for (int k = 0; k < NIN; ++k) Xo[k] = x[k];
-  float* To = lp.T + tid * NT;
-  double defl = 0.0, tilt = 0.0;
-  if (ok) {
-    const double xh[3] = {pos[0] / rpos, pos[1] / rpos, pos[2] / rpos};
-    const double dex[3] = {vel[0] / vl, vel[1] / vl, vel[2] / vl};
-    plane_angles(xh, d0, dex, &defl, &tilt);
-  }
-  To[0] = (float)defl;
-  To[1] = (float)tilt;
-  To[2] = 0.f;
-  To[3] = (r_cross > 0.f ? fminf(10.f / r_cross, 5.f) : 0.f) - 1.f;  // 10/s - 1; no crossing = s -> inf
-  To[4] = r_cross > 0.f ? g_cross - 1.f : 0.f;
-  To[5] = ok ? 1.f : 0.f;
-  To[6] = r_cross > 0.f ? 1.f : 0.f;
-  To[7] = 0.f;
-  if (lp.raw) {
-    float* Ro = lp.raw + tid * NRAW;
-    Ro[0] = (float)r; Ro[1] = (float)th; Ro[2] = (float)a;
-    Ro[3] = nf[0]; Ro[4] = nf[1]; Ro[5] = nf[2];
-    Ro[6] = (float)flags; Ro[7] = (float)steps;
-    Ro[8] = (float)(vel[0] / vl); Ro[9] = (float)(vel[1] / vl); Ro[10] = (float)(vel[2] / vl);
-    Ro[11] = r_cross;
-    Ro[12] = (float)d0[0]; Ro[13] = (float)d0[1]; Ro[14] = (float)d0[2];
-  }
+  label_write(lp, tid, L, y, flags, steps, crossed, c);
 }
 
 // ---------------------------------------------------------------------------
@@ -1355,6 +1634,9 @@ struct st_surrogate {
   // forward epilogues) and dZ (ping-pong, written by the input-gradient epilogues)
   __nv_bfloat16* HT[3] = {nullptr, nullptr, nullptr};
   __nv_bfloat16* dZT[2] = {nullptr, nullptr};
+  unsigned* d_queue = nullptr;  // head of the label kernel's sample queue, and label_order's two histograms
+  uint32_t* d_order = nullptr;  // label_order's rows
+  int order_cap = 0;
   int* d_status = nullptr;                              // tcgen05 GEMM: a bounded wait ran out
   unsigned char* Wsw = nullptr;  // hidden layers as swizzled bf16 images for the tcgen05 frame kernel
   float* Psmall = nullptr;       // FP32 edge layers and biases packed for the same kernel
@@ -1569,6 +1851,31 @@ int backward(st_surrogate* s, const float* X, int B) {
   return l0_backward(s, dZ, X, B, nred);
 }
 
+// The order in which the label kernel takes the last samples of a set: longest
+// rays first, over at most ORDER_MAX rows (4 MB, kept with the object).  A set
+// larger than that spends its time before them.
+int label_order(st_surrogate* s, LabelParams* lp) {
+  const int m = (int)std::min(lp->n, ORDER_MAX);
+  if (s->order_cap < m) {
+    cudaFree(s->d_order);
+    s->d_order = nullptr;
+    s->order_cap = 0;
+    if (cudaMalloc(&s->d_order, (size_t)m * sizeof(uint32_t)) != cudaSuccess) return ST_ENOMEM;
+    s->order_cap = m;
+  }
+  const long long first = lp->n - m;
+  const unsigned nb = (unsigned)((m + 255) / 256);
+  unsigned* hist = s->d_queue + 1;
+  SC(cudaMemsetAsync(s->d_queue, 0, (1 + 2 * ORDER_BUCKETS) * sizeof(unsigned), s->stream));
+  label_count<<<nb, 256, 0, s->stream>>>(first, lp->offset, m, hist);
+  SC(cudaGetLastError());
+  label_place<<<nb, 256, 0, s->stream>>>(first, lp->offset, m, hist, hist + ORDER_BUCKETS, s->d_order);
+  SC(cudaGetLastError());
+  lp->order = s->d_order;
+  lp->sorted = m;
+  return ST_OK;
+}
+
 int pad128(long long n) { return (int)((n + 127) / 128 * 128); }
 
 // After a sync: ST_ECUDA (and the flag cleared) when a tcgen05 GEMM's bounded
@@ -1646,6 +1953,7 @@ int st_surrogate_create(st_surrogate** out, int device, unsigned long long seed)
       return fail(ST_ENOMEM);
   if (cudaMalloc(&s->d_status, sizeof(int)) != cudaSuccess || cudaMemset(s->d_status, 0, sizeof(int)) != cudaSuccess)
     return fail(ST_ENOMEM);
+  if (cudaMalloc(&s->d_queue, (1 + 2 * ORDER_BUCKETS) * sizeof(unsigned)) != cudaSuccess) return fail(ST_ENOMEM);
   if (cudaMalloc(&s->Wsw, TC_WSW_BYTES) != cudaSuccess) return fail(ST_ENOMEM);
   if (cudaMalloc(&s->Psmall, TC_SMALL_BYTES) != cudaSuccess) return fail(ST_ENOMEM);
   // He-style uniform initialisation from a splitmix64 stream (host)
@@ -1688,6 +1996,8 @@ void st_surrogate_destroy(st_surrogate* s) {
   cudaFree(s->P); cudaFree(s->G); cudaFree(s->Mm); cudaFree(s->Vv); cudaFree(s->loss);
   for (int l = 0; l < 3; ++l) { cudaFree(s->Wb[l]); cudaFree(s->Wt[l]); }
   cudaFree(s->d_status);
+  cudaFree(s->d_queue);
+  cudaFree(s->d_order);
   for (int l = 0; l < 3; ++l) cudaFree(s->HT[l]);
   for (int l = 0; l < 2; ++l) cudaFree(s->dZT[l]);
   cudaFree(s->part);
@@ -1801,8 +2111,21 @@ int st_surrogate_generate(st_surrogate* s, long long n, long long offset, double
     return ST_ENOMEM;
   float* raw = nullptr;
   if (host_raw && cudaMalloc(&raw, (size_t)n * NRAW * 4) != cudaSuccess) return ST_ENOMEM;
-  LabelParams lp{n, offset, s->DX, s->DT, raw, dt};
-  label_kernel<<<(unsigned)((n + 127) / 128), 128, 0, s->stream>>>(lp);
+  LabelParams lp{n, offset, s->DX, s->DT, raw, dt, nullptr, 0};
+  if (dt >= 1e-5 && dt <= 100.0 && n <= 0x7fffff00ll) {
+    const int rc = label_order(s, &lp);
+    if (rc != ST_OK) { cudaFree(raw); return rc; }
+    // Warps per SM: two per scheduler fill the FP32 pipe; more only make every
+    // step, and so the longest ray, slower (131,072 labels: 24.3 ms with 8 an SM,
+    // 30.7 with 12; 2^20: 127 ms with either), and a small set ends with its
+    // longest ray (65,536 labels: 16.3 ms with 4 an SM, 21.3 with 8).
+    int nsm = 0;
+    SC(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, s->device));
+    const long long warps = std::min((n + 31) / 32, (long long)nsm * (n <= 65536 ? 4 : LABEL_WARPS));
+    label_pairs_kernel<<<(unsigned)warps, 32, 0, s->stream>>>(lp, s->d_queue);
+  } else {
+    label_kernel<<<(unsigned)((n + 127) / 128), 128, 0, s->stream>>>(lp);
+  }
   SC(cudaGetLastError());
   if (host_x) SC(cudaMemcpyAsync(host_x, s->DX, (size_t)n * NIN * 4, cudaMemcpyDeviceToHost, s->stream));
   if (host_t) SC(cudaMemcpyAsync(host_t, s->DT, (size_t)n * NT * 4, cudaMemcpyDeviceToHost, s->stream));

@@ -897,6 +897,52 @@ __device__ __forceinline__ void land_on_sphere(const R* yp, R pt, R M, R a, R h,
   }
 }
 
+// The same from the state before the step alone, in double: y in and out.  Its
+// four stages share one copy of the right-hand side, for kernels in which
+// landing is cold code beside a hot loop (unrolled it is 80 KB).
+template <int KERR>
+__device__ __forceinline__ void land_in_step(double* y, double pt, double M, double a, double h, double target) {
+  double y0[6];
+#pragma unroll
+  for (int k = 0; k < 6; ++k) y0[k] = y[k];
+  double ha = 0.0, ga = sqrt(y0[0] * y0[0] + y0[1] * y0[1] + y0[2] * y0[2]) - target, hb = h, gb = 0.0, hc = h;
+  int side = 0;
+#pragma unroll 1
+  for (int it = 0; it <= 60; ++it) {
+    // it = 0: the whole step, the bracket's other end
+    if (it > 0) {
+      hc = (ha * gb - hb * ga) / (gb - ga);
+      if (!(hc > ha && hc < hb)) hc = 0.5 * (ha + hb);
+    }
+    double sum[6] = {0, 0, 0, 0, 0, 0};
+#pragma unroll
+    for (int k = 0; k < 6; ++k) y[k] = y0[k];
+#pragma unroll 1
+    for (int s = 0; s < 4; ++s) {
+      double d[6];
+      rhs<KERR>(y, pt, M, a, d);
+      const double w = (s == 1 || s == 2) ? 2.0 : 1.0, c = s < 2 ? 0.5 * hc : hc;
+#pragma unroll
+      for (int k = 0; k < 6; ++k) { sum[k] += w * d[k]; y[k] = y0[k] + c * d[k]; }
+    }
+#pragma unroll
+    for (int k = 0; k < 6; ++k) y[k] = y0[k] + hc / 6.0 * sum[k];
+    const double gc = sqrt(y[0] * y[0] + y[1] * y[1] + y[2] * y[2]) - target;
+    if (it == 0) { gb = gc; continue; }
+    if (gc == 0.0 || (hb - ha) < 1e-15 * h) break;
+    if ((gc > 0.0) == (gb > 0.0)) {
+      hb = hc; gb = gc;
+      if (side == -1) ga *= 0.5;
+      side = -1;
+    } else {
+      ha = hc; ga = gc;
+      if (side == 1) gb *= 0.5;
+      side = 1;
+    }
+    if (fabs(gc) < 1e-14) break;
+  }
+}
+
 // ---- shading pieces applied at interpolated points --------------------------
 
 template <typename R>

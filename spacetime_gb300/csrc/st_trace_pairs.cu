@@ -16,11 +16,13 @@
 namespace st {
 namespace {
 
-using dfm::f3;
+using dfm::dbl;
+using dfm::doubles;
+using dfm::fst;
+using dfm::pair_of;
+using dfm::snd;
 using dfm::t3;
 using dfm::two;
-using dfm::fst;
-using dfm::snd;
 
 struct PairRay {
   t3 P, Q, W;  // (x, y), (p_x, p_y), (z, p_z)
@@ -61,19 +63,6 @@ struct GasWarp {
   df2 r_prev0[32];
   int steps0[32], flags0[32];
 };
-
-__device__ __forceinline__ df2 pair_of(double v) {
-  const float h = (float)v;
-  return df2{h, (float)(v - (double)h)};
-}
-__device__ __forceinline__ double dbl(df2 x) { return (double)x.hi + (double)x.lo; }
-__device__ __forceinline__ double dbl(const f3& x) { return (double)x.h + ((double)x.m + (double)x.l); }
-__device__ __forceinline__ f3 f3_of(double v) {
-  const float h = (float)v;
-  const double r = v - (double)h;
-  const float m = (float)r;
-  return f3{h, m, (float)(r - (double)m)};
-}
 
 __device__ __forceinline__ float2 f2(df2 x) { return make_float2(x.hi, x.lo); }
 __device__ __forceinline__ df2 d2(float2 x) { return df2{x.x, x.y}; }
@@ -208,15 +197,7 @@ __device__ __forceinline__ void mark_ray(const PairRay& st, GasWarp& g, int lane
   g.flags0[lane] = st.flags;
 }
 
-__device__ __forceinline__ void doubles(const t3& P, const t3& Q, const t3& W, double* y) {
-  y[0] = dbl(fst(P)); y[1] = dbl(snd(P)); y[2] = dbl(fst(W));
-  y[3] = dbl(fst(Q)); y[4] = dbl(snd(Q)); y[5] = dbl(snd(W));
-}
-__device__ __forceinline__ void set_state(const double* y, PairRay& st) {
-  st.P = two(f3_of(y[0]), f3_of(y[1]));
-  st.Q = two(f3_of(y[3]), f3_of(y[4]));
-  st.W = two(f3_of(y[2]), f3_of(y[5]));
-}
+__device__ __forceinline__ void set_state(const double* y, PairRay& st) { dfm::set_state(y, &st.P, &st.Q, &st.W); }
 
 // The disc where a step crosses z = 0, in double as in step_ray; P, Q, W the
 // state before the step, st the state after it.
@@ -240,56 +221,6 @@ __device__ __forceinline__ void cross_pairs(const TraceParams& p, const t3& P, c
     st.g_cross = (float)g;
     st.flags |= ST_RAY_CROSSED;
   }
-}
-
-// The state where the ray's last step (from st, of size st.land_h) meets the
-// sphere |x| = target, in double.  Called after the integration loop, for all
-// rays of the warp together: inside it each ray lands at a step of its own, and
-// the landing's double code took a third of the kernel's time.
-// (land_on_sphere's iteration; its four stages share one copy of the double
-// right-hand side, which unrolled is 80 KB of code that every ray runs once.)
-template <int KERR>
-__device__ __forceinline__ void land_pairs(const TraceParams& p, double target, PairRay& st) {
-  double y0[6], y[6];
-  doubles(st.P, st.Q, st.W, y0);
-  const double pt = dbl(st.pt), h = dbl(st.land_h);
-  double ha = 0.0, ga = sqrt(y0[0] * y0[0] + y0[1] * y0[1] + y0[2] * y0[2]) - target, hb = h, gb = 0.0, hc = h;
-  int side = 0;
-#pragma unroll 1
-  for (int it = 0; it <= 60; ++it) {
-    // it = 0: the whole step, the bracket's other end
-    if (it > 0) {
-      hc = (ha * gb - hb * ga) / (gb - ga);
-      if (!(hc > ha && hc < hb)) hc = 0.5 * (ha + hb);
-    }
-    double sum[6] = {0, 0, 0, 0, 0, 0};
-#pragma unroll
-    for (int k = 0; k < 6; ++k) y[k] = y0[k];
-#pragma unroll 1
-    for (int s = 0; s < 4; ++s) {
-      double d[6];
-      rhs<KERR>(y, pt, p.M, p.a, d);
-      const double w = (s == 1 || s == 2) ? 2.0 : 1.0, c = s < 2 ? 0.5 * hc : hc;
-#pragma unroll
-      for (int k = 0; k < 6; ++k) { sum[k] += w * d[k]; y[k] = y0[k] + c * d[k]; }
-    }
-#pragma unroll
-    for (int k = 0; k < 6; ++k) y[k] = y0[k] + hc / 6.0 * sum[k];
-    const double gc = sqrt(y[0] * y[0] + y[1] * y[1] + y[2] * y[2]) - target;
-    if (it == 0) { gb = gc; continue; }
-    if (gc == 0.0 || (hb - ha) < 1e-15 * h) break;
-    if ((gc > 0.0) == (gb > 0.0)) {
-      hb = hc; gb = gc;
-      if (side == -1) ga *= 0.5;
-      side = -1;
-    } else {
-      ha = hc; ga = gc;
-      if (side == 1) gb *= 0.5;
-      side = 1;
-    }
-    if (fabs(gc) < 1e-14) break;
-  }
-  set_state(y, st);
 }
 
 // The tests of step_ray before a step (capture, escape, budget) and the step's
@@ -333,41 +264,22 @@ __device__ __forceinline__ bool begin_pairs(const TraceParams& p, const dfm::Geo
 }
 
 // One step of step_ray's rules (RK4); true when the ray is done.  The four
-// stages share one copy of the right-hand side: unrolled, the step and the gas
+// stages share one copy of the right-hand side (dfm::rk4): unrolled, the step and the gas
 // sample outgrow the instruction caches (4.8 of 7 stall cycles an instruction
 // were fetches, and the 320x180 gas frame took 34.7 ms, rolled 25.2).
 template <int KERR, int VOL, int SEM>
 __device__ __forceinline__ bool step_pairs(const TraceParams& p, PairRay& st, GasWarp* gas, int lane) {
   using namespace dfm;
   const Scene& C = p.d;
-  const Hole& H = C.H;
   if (st.steps >= st.nmax) { st.flags |= ST_RAY_BUDGET; return true; }
   df2 h, r2, v2;
-  dd tP = top(st.P), tQ = top(st.Q), tW = top(st.W);
-  dd iP = two(q(0.f), q(0.f)), iQ = iP, iW = iP;
-#pragma unroll 1
-  for (int s = 0; s < 4; ++s) {
-    const Geo g = geometry<KERR>(tP, fst(tW), H);
-    if (s == 0) {
-      if (begin_pairs<KERR, VOL, SEM>(p, g, st, &h)) return true;
-      r2 = g.flat2;
-    }
-    dd kP, kQ, kW;
-    rhs<KERR>(tP, tQ, tW, g, st.pt, H, &kP, &kQ, &kW);
-    if (VOL && s == 0) v2 = sumsq(fst(kP), snd(kP), fst(kW), q(0.f));
-    const float w = (s == 1 || s == 2) ? 2.f : 1.f;
-    iP = add(iP, scale(kP, w));
-    iQ = add(iQ, scale(kQ, w));
-    iW = add(iW, scale(kW, w));
-    const dd hs = both(scale(h, s < 2 ? 0.5f : 1.f));
-    tP = fma1(hs, kP, top(st.P));
-    tQ = fma1(hs, kQ, top(st.Q));
-    tW = fma1(hs, kW, top(st.W));
-  }
-  const dd h6 = both(mul(h, df2{0.166666672f, -4.96705388e-9f}));
-  iP = mul(h6, iP);
-  iQ = mul(h6, iQ);
-  iW = mul(h6, iW);
+  dd iP, iQ, iW;
+  const bool done = rk4<KERR>(
+      st.P, st.Q, st.W, st.pt, C.H,
+      [&](const Geo& g, df2* hh) { r2 = g.flat2; return begin_pairs<KERR, VOL, SEM>(p, g, st, hh); },
+      [&](const dd& kP, const dd& kW) { if (VOL) v2 = sumsq(fst(kP), snd(kP), fst(kW), q(0.f)); },
+      &h, &iP, &iQ, &iW);
+  if (done) return true;
   const t3 P = st.P, Q = st.Q, W = st.W;
   st.P = add3(P, iP);
   st.Q = add3(Q, iQ);
@@ -502,10 +414,13 @@ __global__ void __launch_bounds__(PAIR_BLOCK, ST_PAIR_MINB) trace_pairs_kernel(c
   }
   unsigned long long steps = 0, gas = 0, rays = 0;
   if (live) {
-    if (st.land_h.hi > 0.f)
-      land_pairs<KERR>(p, SEM == ST_SEM_RENDER && (st.flags & ST_RAY_CAPTURED) ? 2.00001 : dbl(st.r_esc), st);
     RayState<double> s1;
     doubles(st.P, st.Q, st.W, s1.y);
+    // after the loop, for all rays of the warp together: inside it each ray lands
+    // at a step of its own, and that double code took a third of the kernel's time
+    if (st.land_h.hi > 0.f)
+      land_in_step<KERR>(s1.y, dbl(st.pt), p.M, p.a, dbl(st.land_h),
+                         SEM == ST_SEM_RENDER && (st.flags & ST_RAY_CAPTURED) ? 2.00001 : dbl(st.r_esc));
     s1.pt = dbl(st.pt);
     s1.scam = dbl(st.scam);
 #pragma unroll

@@ -72,23 +72,17 @@ static void step(T* y, T pt, T a) {
 
 template <int KERR>
 static void step_pairs(D::t3* P, D::t3* Qm, D::t3* W, df2 pt, const D::Hole& H) {
-  dd tP = D::top(*P), tQ = D::top(*Qm), tW = D::top(*W), iP = D::two(D::q(0), D::q(0)), iQ = iP, iW = iP;
-  df2 h{0, 0};
-  for (int s = 0; s < 4; ++s) {
-    const D::Geo g = D::geometry<KERR>(tP, D::fst(tW), H);
-    if (!s) {
-      const df2 c = D::mul(pair((Q)0.16), D::sqrt_(g.flat2));
-      h = D::mul(pair((Q)0.02), D::min_(D::max_(c, D::q(1)), D::q(8)));
-    }
-    dd kP, kQ, kW;
-    D::rhs<KERR>(tP, tQ, tW, g, pt, H, &kP, &kQ, &kW);
-    const float w = (s == 1 || s == 2) ? 2.f : 1.f;
-    iP = D::add(iP, D::scale(kP, w)); iQ = D::add(iQ, D::scale(kQ, w)); iW = D::add(iW, D::scale(kW, w));
-    const dd hs = D::both(D::scale(h, s < 2 ? 0.5f : 1.f));
-    tP = D::fma1(hs, kP, D::top(*P)); tQ = D::fma1(hs, kQ, D::top(*Qm)); tW = D::fma1(hs, kW, D::top(*W));
-  }
-  const dd h6 = D::both(D::mul(h, pair(Q(1) / 6)));
-  *P = D::add3(*P, D::mul(h6, iP)); *Qm = D::add3(*Qm, D::mul(h6, iQ)); *W = D::add3(*W, D::mul(h6, iW));
+  dd iP, iQ, iW;
+  df2 h;
+  D::rk4<KERR>(
+      *P, *Qm, *W, pt, H,
+      [](const D::Geo& g, df2* hh) {
+        const df2 c = D::mul(pair((Q)0.16), D::sqrt_(g.flat2));
+        *hh = D::mul(pair((Q)0.02), D::min_(D::max_(c, D::q(1)), D::q(8)));
+        return false;
+      },
+      [](const dd&, const dd&) {}, &h, &iP, &iQ, &iW);
+  *P = D::add3(*P, iP); *Qm = D::add3(*Qm, iQ); *W = D::add3(*W, iW);
 }
 
 static double U() { return (rand() + rand() / (RAND_MAX + 1.0)) / (RAND_MAX + 1.0); }

@@ -70,3 +70,16 @@ def test_outside_the_rule_the_double_kernel_runs(built_lib):
         a_, b_ = _both(ctx, cam, Schwarzschild(M), _abi.ST_SEM_DRAFT, width=16, height=9, samples=1, pixel_jitter=0,
                        dt=0.05 * M, nmax=4000)
     _same(a_, b_)
+
+
+def test_labels_do_not_depend_on_the_queue(built_lib):
+    """Every row is written, whatever the set's size (below a warp, ragged, on
+    either side of the warp-count rule) and the order its rays are taken in: a
+    row has the same bits in every set that holds it."""
+    from spacetime_gb300.surrogate import Surrogate
+    s = Surrogate()
+    big = s.generate(66001, offset=5)
+    for n, off in ((1, 5), (31, 5), (33, 17), (1000, 60005), (65536, 5), (65537, 300)):
+        for a_, b_ in zip(s.generate(n, offset=off), big):
+            assert np.isfinite(a_).all() and np.array_equal(a_, b_[off - 5:off - 5 + n])
+    s.close()
