@@ -89,18 +89,17 @@ enum { ST_EMIT_KEPLER = 0, ST_EMIT_KS_EXACT = 1 };
 enum { ST_SEM_RENDER = 0, ST_SEM_DRAFT = 1 };
 /* arithmetic of the geodesic integration */
 enum {
-  ST_PREC_FP64 = 0,          /* everything in double */
+  ST_PREC_FP64 = 0,          /* double accuracy: everything in double, or (RK4
+                                frames of the pixel schedule) slopes in pairs
+                                of floats and the state in three, whose error
+                                against the exact RK4 sequence is smaller */
   ST_PREC_FP32_GUARDED = 1,  /* FP32 RK4 with a compensated (float-float) state;
-                                FP64 for steps inside r_guard, for rays in the
-                                critical band, and for the null-constraint
-                                renormalisation */
+                                steps inside r_guard, of rays in the critical
+                                band, and the null-constraint renormalisation
+                                at the state's full 48 bits (float pairs) */
   ST_PREC_FP32 = 2,          /* plain FP32, as the reference's Metal kernel */
-  ST_PREC_FP32_GUARDED_DF = 3  /* ST_PREC_FP32_GUARDED with the guard steps and
-                                the null renormalisation in double-float
-                                arithmetic (pairs of floats, about 47-bit
-                                significands) on the FP32 pipe instead of
-                                FP64, whose rate on GB300 is a small fraction
-                                of FP32's */
+  ST_PREC_FP32_GUARDED_DF = 3  /* the same kernels as ST_PREC_FP32_GUARDED
+                                (whose guard steps were once in double) */
 };
 /* launch schedule */
 enum {
@@ -179,13 +178,13 @@ typedef struct {
   int exit_landing;          /* land exactly on r_escape before reading the sky */
   int pixel_jitter;          /* per-pixel hashed jitter inside each stratum */
   unsigned long long seed;   /* pass shuffles and hash seeds */
-  double r_guard;            /* FP32_GUARDED: FP64 steps inside this KS radius
+  double r_guard;            /* FP32_GUARDED: guard steps inside this KS radius
                                 (rays not already proven captured); 0 = off */
-  double crit_band;          /* FP32_GUARDED: critical-band rays get FP64 steps:
+  double crit_band;          /* FP32_GUARDED: critical-band rays get guard steps:
                                 |b - b_crit| < crit_band (Schwarzschild) or the
                                 Bardeen graze flag (Kerr); <= 0 = off */
   double crit_r;             /* ...but only inside this KS radius; 0 = whole ray */
-  int renorm_every;          /* FP32_GUARDED: FP64 null renormalisation period; 0 = off */
+  int renorm_every;          /* FP32_GUARDED: null renormalisation period; 0 = off */
   int surrogate;             /* 1 = gate + learned surrogate (st_surrogate_*) */
   double surrogate_sigma;    /* gate: max predicted std-dev (rad) served */
   int block_x, block_y;      /* ST_SCHED_PIXEL tile; 0 = tuned default */

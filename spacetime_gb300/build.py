@@ -20,7 +20,7 @@ LIB = os.environ.get("SPACETIME_GB300_LIB", os.path.join(HERE, "libspacetime_gb3
 # resident blocks per SM to keep FP32 latency hidden
 FAST = os.environ.get("ST_FASTMATH", "1") == "1"
 MINB_FP32 = os.environ.get("ST_MINB_FP32", "7")
-MINB_FP32G = os.environ.get("ST_MINB_FP32G", "4")
+MINB_FP32G = os.environ.get("ST_MINB_FP32G", "5")
 MINB_FP64 = os.environ.get("ST_MINB_FP64", "1")
 MINB_PAIRS = os.environ.get("ST_MINB_PAIRS", "12")
 UNIT_FLAGS = {

@@ -551,9 +551,8 @@ int fill_params(st_context* ctx, const st_camera* cam, const st_spacetime* stp, 
   p->queue = ctx->d_queue;
   p->chunk_steps = rp->chunk_steps > 0 ? rp->chunk_steps : 32;
   p->refill_window = refill_window();
-  // double-float guards run in the FP32_GUARDED kernels
+  // both guarded precisions run the same kernels: their guard steps are float pairs
   v->prec = rp->precision == ST_PREC_FP32_GUARDED_DF ? ST_PREC_FP32_GUARDED : rp->precision;
-  p->guard_df = rp->precision == ST_PREC_FP32_GUARDED_DF ? 1 : 0;
   v->kerr = (a != 0.0) ? 1 : 0;
   v->vol = p->vol_on;
   v->sem = rp->semantics;
@@ -1807,7 +1806,6 @@ int fill_frame_params(const st_camera* cam, const st_spacetime* stp, const st_re
   p->crit_r2 = rp->crit_r > 0.0 ? rp->crit_r * rp->crit_r : 0.0;
   p->b_crit = 3.0 * std::sqrt(3.0) * M;
   p->renorm_every = rp->renorm_every;
-  p->guard_df = rp->precision == ST_PREC_FP32_GUARDED_DF ? 1 : 0;
   p->refill_window = 32;
   p->chunk_steps = rp->chunk_steps > 0 ? rp->chunk_steps : 32;
   return ST_OK;

@@ -10,8 +10,9 @@
 // Precision:
 //   ST_PREC_FP64          all double
 //   ST_PREC_FP32          all float (the reference kernel's arithmetic)
-//   ST_PREC_FP32_GUARDED  float RHS, float-float (TwoSum) state, FP64 steps
-//                         for guarded rays/regions, FP64 null renormalisation
+//   ST_PREC_FP32_GUARDED  float RHS, float-float (TwoSum) state, float-pair
+//                         steps for guarded rays/regions, and the same for the
+//                         null renormalisation
 #pragma once
 
 #include <cuda_runtime.h>
@@ -180,44 +181,6 @@ __device__ __forceinline__ void rhs_kerr_f32(const float* s, float pt, float M, 
   d[3] = fmaf(Gr, x, fmaf(Fr, px, -(Fa * py)));
   d[4] = fmaf(Gr, y, fmaf(Fr, py, Fa * px));
   d[5] = fmaf(z * isig, fmaf(G * r, r2a, -((a2 * ell) * fl)), flir * pz);
-}
-
-// The regrouped Kerr RHS above in double, for the FP32_GUARDED path's FP64
-// guard steps: the same algebra (r from the half-w quartic root, one
-// reciprocal square root for r and 1/r, two reciprocals), so a guard step
-// issues about half the FP64 instructions of the term-by-term form.  On GB300
-// an FP64 instruction costs tens of FP32 ones; the all-FP64 precision keeps
-// the term-by-term form the oracle restates.
-__device__ __forceinline__ void rhs_kerr_rg64(const double* s, double pt, double M, double a, double* d) {
-  const double x = s[0], y = s[1], z = s[2], px = s[3], py = s[4], pz = s[5];
-  const double a2 = a * a, z2 = z * z;
-  const double q = a2 * z2;
-  const double wh = fma(fma(x, x, fma(y, y, z2)), 0.5, -(0.5 * a2));
-  const double r2 = fmax(wh + sqrt(fma(wh, wh, q)), 1e-12);
-  const double ir = rsqrt(r2), r = r2 * ir;
-  const double isig = 1.0 / fma(r2, r2, q);
-  const double r2a = r2 + a2;
-  const double ira = 1.0 / r2a;
-  const double A = fma(px, x, py * y);
-  const double B = fma(px, y, -(py * x));
-  const double T = fma(r, A, a * B) * ira;
-  const double Z = (z * pz) * ir;
-  const double ell = (T + Z) - pt;
-  const double rsig = (r2 * r) * isig;
-  const double fl = ((2.0 * M) * rsig) * ell;
-  const double Fi = fl * ira;
-  const double Fr = Fi * r, Fa = Fi * a;
-  const double flir = fl * ir;
-  d[0] = fma(-Fr, x, fma(-Fa, y, px));
-  d[1] = fma(-Fr, y, fma(Fa, x, py));
-  d[2] = fma(-flir, z, pz);
-  const double dldr = fma(fma(-2.0 * r, T, A), ira, -(Z * ir));
-  const double inner = fma(ell * ir, fma(q + q, isig, -0.5), dldr);
-  const double G = fl * inner;
-  const double Gr = G * rsig;
-  d[3] = fma(Gr, x, fma(Fr, px, -(Fa * py)));
-  d[4] = fma(Gr, y, fma(Fr, py, Fa * px));
-  d[5] = fma(z * isig, fma(G * r, r2a, -((a2 * ell) * fl)), flir * pz);
 }
 
 // Kerr, src/metal.jl:466-508 (implicit-quartic r, four derivative terms).
@@ -1077,36 +1040,6 @@ __device__ __forceinline__ bool march_gas(const TraceParams& p, const R* yp, con
   return st.alpha < R(0.003);
 }
 
-// Null-constraint renormalisation in FP64: rescale the spatial momentum so
-// that H = 1/2(-p_t^2 + |p|^2 - f l^2) = 0 at fixed p_t.
-template <int KERR>
-__device__ __forceinline__ void null_renorm(double* y, double pt, double M, double a) {
-  double f, L[3];
-  if constexpr (KERR) {
-    const double a2 = a * a;
-    const double r2 = fmax(ks_r2(y[0], y[1], y[2], a), 1e-12);
-    const double r = sqrt(r2);
-    const double ira = 1.0 / (r2 + a2);
-    L[0] = (r * y[0] + a * y[1]) * ira;
-    L[1] = (r * y[1] - a * y[0]) * ira;
-    L[2] = y[2] / r;
-    f = 2.0 * M * r2 * r / (r2 * r2 + a2 * y[2] * y[2]);
-  } else {
-    const double r = sqrt(y[0] * y[0] + y[1] * y[1] + y[2] * y[2]);
-    L[0] = y[0] / r; L[1] = y[1] / r; L[2] = y[2] / r;
-    f = 2.0 * M / r;
-  }
-  const double kap = L[0] * y[3] + L[1] * y[4] + L[2] * y[5];
-  const double pp = y[3] * y[3] + y[4] * y[4] + y[5] * y[5];
-  const double A = pp - f * kap * kap;
-  const double B = 2.0 * f * pt * kap;
-  const double C = -(1.0 + f) * pt * pt;
-  const double disc = B * B - 4.0 * A * C;
-  if (!(A > 0.0) || !(disc >= 0.0)) return;
-  const double lam = (-B + sqrt(disc)) / (2.0 * A);
-  if (lam > 0.9 && lam < 1.1) { y[3] *= lam; y[4] *= lam; y[5] *= lam; }
-}
-
 // Tsitouras (2011) 5(4) pair, FSAL (published tableau).
 struct Tsit5C {
   static constexpr double A21 = 0.161;
@@ -1183,245 +1116,66 @@ __device__ __forceinline__ R tsit5_adaptive(const R* s0, R pt, R M, R a, R r, R 
   return h_used;
 }
 
-// RHS of the guard steps: the regrouped Kerr form in double, Schwarzschild as is.
+// The guarded path's guard step and null renormalisation, on its float-float
+// state, in the float pairs of st_df.cuh.  The state holds 48 bits whatever the
+// step is computed in: in double and in pairs the exit directions of fully
+// guarded rays are off by the same 3.2e-14 to 3.7e-14 (median over cameras and
+// spins, against 128-bit arithmetic), which is the state's own rounding.  A
+// double guard step held its whole warp for about 5,900 cycles of the SM's FP64
+// pipe, and the frame ended on the rays that are guarded all the way: 960x540
+// Kerr gas at the default guards, 86-101 ms with double steps, 26.1 with an
+// earlier double-float step, 20.8 ms now; 1080p 134 -> 58.9 ms.
 template <int KERR>
-__device__ __forceinline__ void rhs_guard(const double* s, double pt, double M, double a, double* d) {
-  if constexpr (KERR) rhs_kerr_rg64(s, pt, M, a, d); else rhs_schw(s, pt, M, d);
+__device__ __forceinline__ void guard_step(float* y, float* lo, float pt, const TraceParams& p, float h) {
+  using namespace dfm;
+  const v2 zero = mkv(0.f, 0.f);
+  t3 P{mkv(y[0], y[1]), mkv(lo[0], lo[1]), zero}, Q{mkv(y[3], y[4]), mkv(lo[3], lo[4]), zero};
+  t3 W{mkv(y[2], y[5]), mkv(lo[2], lo[5]), zero};
+  df2 hh;
+  dd iP, iQ, iW;
+  rk4<KERR>(
+      P, Q, W, q(pt), p.d.H, [&](const Geo&, df2* o) { *o = q(h); return false; }, [](const dd&, const dd&) {}, &hh,
+      &iP, &iQ, &iW);
+  const dd a = add(top(P), iP), b = add(top(Q), iQ), c = add(top(W), iW);
+  y[0] = a.h.x; y[1] = a.h.y; lo[0] = a.l.x; lo[1] = a.l.y;
+  y[3] = b.h.x; y[4] = b.h.y; lo[3] = b.l.x; lo[4] = b.l.y;
+  y[2] = c.h.x; y[5] = c.h.y; lo[2] = c.l.x; lo[5] = c.l.y;
 }
 
-// FP64 guard step on the float-float state (classical RK4 in double).
+// Null-constraint renormalisation: rescale the spatial momentum so that
+// H = 1/2(-p_t^2 + |p|^2 - f l^2) = 0 at fixed p_t.
 template <int KERR>
-__device__ __forceinline__ void guard_step_fp64(float* y, float* lo, float pt, double M, double a, float h) {
-  double yd[6], k1d[6], inc[6];
-#pragma unroll
-  for (int k = 0; k < 6; ++k) yd[k] = (double)y[k] + (double)lo[k];
-  const double ptd = (double)pt;
-  rhs_guard<KERR>(yd, ptd, M, a, k1d);
-  {
-    double t[6], k[6], sum[6];
-    const double hd = (double)h, hh = 0.5 * hd;
-#pragma unroll
-    for (int i = 0; i < 6; ++i) { t[i] = fma(hh, k1d[i], yd[i]); sum[i] = k1d[i]; }
-    rhs_guard<KERR>(t, ptd, M, a, k);
-#pragma unroll
-    for (int i = 0; i < 6; ++i) { sum[i] = fma(2.0, k[i], sum[i]); t[i] = fma(hh, k[i], yd[i]); }
-    rhs_guard<KERR>(t, ptd, M, a, k);
-#pragma unroll
-    for (int i = 0; i < 6; ++i) { sum[i] = fma(2.0, k[i], sum[i]); t[i] = fma(hd, k[i], yd[i]); }
-    rhs_guard<KERR>(t, ptd, M, a, k);
-    const double h6 = hd * (1.0 / 6.0);
-#pragma unroll
-    for (int i = 0; i < 6; ++i) inc[i] = h6 * (sum[i] + k[i]);
-  }
-#pragma unroll
-  for (int k = 0; k < 6; ++k) {
-    const double v = yd[k] + inc[k];
-    const float hi = (float)v;
-    y[k] = hi;
-    lo[k] = (float)(v - (double)hi);
-  }
-}
-
-// ---------------------------------------------------------------------------
-// Double-float arithmetic on the FP32 pipe (ST_PREC_FP32_GUARDED_DF): a value
-// is hi + lo, two floats with |lo| <= ulp(hi) / 2, about 48 significant bits.
-// Sums by Knuth's TwoSum and Dekker's FastTwoSum, products by the exact FMA
-// residual, reciprocal and (reciprocal) square roots by one Newton-Raphson
-// step from the float value (which doubles its ~23 correct bits).  Every
-// operation is a rounded intrinsic, so neither contraction nor fast-math
-// flags of the translation unit change the error-free transformations.
-// ---------------------------------------------------------------------------
-__device__ __forceinline__ df2 dfq(float a) { return df2{a, 0.f}; }
-__device__ __forceinline__ df2 df_two_sum(float a, float b) {
-  const float s = __fadd_rn(a, b);
-  const float bb = __fsub_rn(s, a);
-  return df2{s, __fadd_rn(__fsub_rn(a, __fsub_rn(s, bb)), __fsub_rn(b, bb))};
-}
-// |a| >= |b| (or a = 0)
-__device__ __forceinline__ df2 df_fast(float a, float b) {
-  const float s = __fadd_rn(a, b);
-  return df2{s, __fsub_rn(b, __fsub_rn(s, a))};
-}
-// x + y with one TwoSum on the high parts and the low parts added in float
-// (Dekker's add): the error is about 2^-47 of max(|x|, |y|) -- an absolute
-// bound at the operands' scale, which is what a guard step's state needs --
-// for half the instructions of the form that also bounds it relative to the
-// sum under cancellation
-__device__ __forceinline__ df2 df_add(df2 x, df2 y) {
-  const df2 s = df_two_sum(x.hi, y.hi);
-  return df_fast(s.hi, __fadd_rn(s.lo, __fadd_rn(x.lo, y.lo)));
-}
-__device__ __forceinline__ df2 df_neg(df2 x) { return df2{-x.hi, -x.lo}; }
-__device__ __forceinline__ df2 df_sub(df2 x, df2 y) { return df_add(x, df_neg(y)); }
-__device__ __forceinline__ df2 df_mul(df2 x, df2 y) {
-  const float p = __fmul_rn(x.hi, y.hi);
-  float e = __fmaf_rn(x.hi, y.hi, -p);
-  e = __fmaf_rn(x.hi, y.lo, e);
-  e = __fmaf_rn(x.lo, y.hi, e);
-  return df_fast(p, e);
-}
-__device__ __forceinline__ df2 df_mulf(df2 x, float f) {
-  const float p = __fmul_rn(x.hi, f);
-  return df_fast(p, __fmaf_rn(x.lo, f, __fmaf_rn(x.hi, f, -p)));
-}
-// x y + z
-__device__ __forceinline__ df2 df_fma(df2 x, df2 y, df2 z) { return df_add(df_mul(x, y), z); }
-// 1 / x: r0 + r0 (1 - x r0)
-__device__ __forceinline__ df2 df_rcp(df2 x) {
-  const float r0 = __frcp_rn(x.hi);
-  const df2 e = df_sub(dfq(1.f), df_mulf(x, r0));
-  return df_fast(r0, __fmul_rn(r0, e.hi));
-}
-// sqrt(x), x > 0: s0 + (x - s0^2) / (2 s0)
-__device__ __forceinline__ df2 df_sqrt(df2 x) {
-  if (!(x.hi > 0.f)) return dfq(0.f);
-  const float s0 = __fsqrt_rn(x.hi);
-  const float p = __fmul_rn(s0, s0);
-  const df2 d = df_sub(x, df2{p, __fmaf_rn(s0, s0, -p)});
-  return df_fast(s0, __fmul_rn(d.hi, __frcp_rn(__fmul_rn(2.f, s0))));
-}
-// 1 / sqrt(x), x > 0: r0 + r0 (1 - x r0^2) / 2
-__device__ __forceinline__ df2 df_rsqrt(df2 x) {
-  const float r0 = __frsqrt_rn(x.hi);
-  const float p = __fmul_rn(r0, r0);
-  const df2 e = df_sub(dfq(1.f), df_mul(x, df2{p, __fmaf_rn(r0, r0, -p)}));
-  return df_fast(r0, __fmul_rn(__fmul_rn(0.5f, r0), e.hi));
-}
-
-// The guard RHS in double-float: the regrouped Kerr form of rhs_kerr_f32 /
-// rhs_kerr_rg64, and the Schwarzschild form of rhs_schw.
-template <int KERR>
-__device__ __forceinline__ void rhs_df(const df2* s, df2 pt, df2 M, df2 a, df2* d) {
-  const df2 x = s[0], y = s[1], z = s[2], px = s[3], py = s[4], pz = s[5];
-  if constexpr (KERR) {
-    const df2 a2 = df_mul(a, a), z2 = df_mul(z, z);
-    const df2 q = df_mul(a2, z2);
-    const df2 wh = df_sub(df_mulf(df_add(df_add(df_mul(x, x), df_mul(y, y)), z2), 0.5f), df_mulf(a2, 0.5f));
-    df2 r2 = df_add(wh, df_sqrt(df_add(df_mul(wh, wh), q)));
-    if (!(r2.hi > 1e-12f)) r2 = dfq(1e-12f);
-    const df2 ir = df_rsqrt(r2), r = df_mul(r2, ir);
-    const df2 isig = df_rcp(df_add(df_mul(r2, r2), q));
-    const df2 r2a = df_add(r2, a2);
-    const df2 ira = df_rcp(r2a);
-    const df2 A = df_add(df_mul(px, x), df_mul(py, y));
-    const df2 B = df_sub(df_mul(px, y), df_mul(py, x));
-    const df2 T = df_mul(df_add(df_mul(r, A), df_mul(a, B)), ira);
-    const df2 Z = df_mul(df_mul(z, pz), ir);
-    const df2 ell = df_sub(df_add(T, Z), pt);
-    const df2 rsig = df_mul(df_mul(r2, r), isig);
-    const df2 fl = df_mul(df_mul(df_mulf(M, 2.f), rsig), ell);
-    const df2 Fi = df_mul(fl, ira);
-    const df2 Fr = df_mul(Fi, r), Fa = df_mul(Fi, a);
-    const df2 flir = df_mul(fl, ir);
-    d[0] = df_sub(df_sub(px, df_mul(Fr, x)), df_mul(Fa, y));
-    d[1] = df_add(df_sub(py, df_mul(Fr, y)), df_mul(Fa, x));
-    d[2] = df_sub(pz, df_mul(flir, z));
-    const df2 dldr = df_sub(df_mul(df_sub(A, df_mul(df_mulf(r, 2.f), T)), ira), df_mul(Z, ir));
-    const df2 inner = df_add(df_mul(df_mul(ell, ir), df_sub(df_mul(df_mulf(q, 2.f), isig), dfq(0.5f))), dldr);
-    const df2 G = df_mul(fl, inner);
-    const df2 Gr = df_mul(G, rsig);
-    d[3] = df_sub(df_add(df_mul(Gr, x), df_mul(Fr, px)), df_mul(Fa, py));
-    d[4] = df_add(df_add(df_mul(Gr, y), df_mul(Fr, py)), df_mul(Fa, px));
-    d[5] = df_add(df_mul(df_mul(z, isig), df_sub(df_mul(df_mul(G, r), r2a), df_mul(df_mul(a2, ell), fl))),
-                  df_mul(flir, pz));
-  } else {
-    const df2 r2 = df_add(df_add(df_mul(x, x), df_mul(y, y)), df_mul(z, z));
-    const df2 ir = df_rsqrt(r2);
-    const df2 f = df_mul(df_mulf(M, 2.f), ir);
-    const df2 kap = df_mul(df_add(df_add(df_mul(x, px), df_mul(y, py)), df_mul(z, pz)), ir);
-    const df2 ell = df_sub(kap, pt);
-    const df2 c1 = df_mul(df_mul(f, ell), ir);
-    const df2 c2 = df_mul(df_mul(c1, df_add(df_mulf(ell, 0.5f), kap)), ir);
-    d[0] = df_sub(px, df_mul(c1, x));
-    d[1] = df_sub(py, df_mul(c1, y));
-    d[2] = df_sub(pz, df_mul(c1, z));
-    d[3] = df_sub(df_mul(c1, px), df_mul(c2, x));
-    d[4] = df_sub(df_mul(c1, py), df_mul(c2, y));
-    d[5] = df_sub(df_mul(c1, pz), df_mul(c2, z));
-  }
-}
-
-// Guard step in double-float on the float-float state (classical RK4).
-template <int KERR>
-__device__ __forceinline__ void guard_step_df(float* y, float* lo, float pt, const TraceParams& p, float h) {
-  df2 Y[6], k1[6], k[6], sum[6], t[6];
-#pragma unroll
-  for (int i = 0; i < 6; ++i) Y[i] = df2{y[i], lo[i]};
-  const df2 PT = dfq(pt), M = df2{p.f.M, p.f.M_lo}, A = df2{p.f.a, p.f.a_lo};
-  const df2 hd = dfq(h), hh = dfq(0.5f * h);
-  rhs_df<KERR>(Y, PT, M, A, k1);
-#pragma unroll
-  for (int i = 0; i < 6; ++i) { t[i] = df_fma(hh, k1[i], Y[i]); sum[i] = k1[i]; }
-  rhs_df<KERR>(t, PT, M, A, k);
-#pragma unroll
-  for (int i = 0; i < 6; ++i) { sum[i] = df_add(sum[i], df_mulf(k[i], 2.f)); t[i] = df_fma(hh, k[i], Y[i]); }
-  rhs_df<KERR>(t, PT, M, A, k);
-#pragma unroll
-  for (int i = 0; i < 6; ++i) { sum[i] = df_add(sum[i], df_mulf(k[i], 2.f)); t[i] = df_fma(hd, k[i], Y[i]); }
-  rhs_df<KERR>(t, PT, M, A, k);
-  const df2 h6 = df_mul(hd, df_rcp(dfq(6.f)));
-#pragma unroll
-  for (int i = 0; i < 6; ++i) {
-    const df2 v = df_add(Y[i], df_mul(h6, df_add(sum[i], k[i])));
-    y[i] = v.hi;
-    lo[i] = v.lo;
-  }
-}
-
-// The null renormalisation (null_renorm) in double-float, for the guarded
-// path's double-float mode.
-template <int KERR>
-__device__ __forceinline__ void renorm_df(float* y, float* lo, float pt, const TraceParams& p) {
+__device__ __forceinline__ void null_renorm(float* y, float* lo, float ptf, const TraceParams& p) {
+  using namespace dfm;
   df2 Y[6];
 #pragma unroll
   for (int i = 0; i < 6; ++i) Y[i] = df2{y[i], lo[i]};
-  const df2 M = df2{p.f.M, p.f.M_lo}, PT = dfq(pt);
-  df2 f, L[3];
+  const Hole& H = p.d.H;
+  const df2 pt = q(ptf);
+  const Geo g = geometry<KERR>(two(Y[0], Y[1]), Y[2], H);
+  df2 f, kap;
   if constexpr (KERR) {
-    const df2 a = df2{p.f.a, p.f.a_lo};
-    const df2 a2 = df_mul(a, a), z2 = df_mul(Y[2], Y[2]), q = df_mul(a2, z2);
-    const df2 wh = df_sub(df_mulf(df_add(df_add(df_mul(Y[0], Y[0]), df_mul(Y[1], Y[1])), z2), 0.5f), df_mulf(a2, 0.5f));
-    df2 r2 = df_add(wh, df_sqrt(df_add(df_mul(wh, wh), q)));
-    if (!(r2.hi > 1e-12f)) r2 = dfq(1e-12f);
-    const df2 ir = df_rsqrt(r2), r = df_mul(r2, ir);
-    const df2 ira = df_rcp(df_add(r2, a2));
-    L[0] = df_mul(df_add(df_mul(r, Y[0]), df_mul(a, Y[1])), ira);
-    L[1] = df_mul(df_sub(df_mul(r, Y[1]), df_mul(a, Y[0])), ira);
-    L[2] = df_mul(Y[2], ir);
-    f = df_mul(df_mul(df_mulf(M, 2.f), df_mul(r2, r)), df_rcp(df_add(df_mul(r2, r2), q)));
+    const df2 ira = rcp(add(g.r2, H.a2));
+    const df2 A = dot2(Y[3], Y[0], Y[4], Y[1]), B = dot2(Y[3], Y[1], neg(Y[4]), Y[0]);
+    kap = fma1(dot2(g.r, A, H.a, B), ira, mul(mul(Y[2], Y[5]), g.ir));
+    f = mul(H.M, mul(g.r, g.iS));
   } else {
-    const df2 ir = df_rsqrt(df_add(df_add(df_mul(Y[0], Y[0]), df_mul(Y[1], Y[1])), df_mul(Y[2], Y[2])));
-    L[0] = df_mul(Y[0], ir); L[1] = df_mul(Y[1], ir); L[2] = df_mul(Y[2], ir);
-    f = df_mul(df_mulf(M, 2.f), ir);
+    kap = mul(dot3(Y[0], Y[3], Y[1], Y[4], Y[2], Y[5]), g.ir);
+    f = mul(scale(H.M, 2.f), g.ir);
   }
-  const df2 kap = df_add(df_add(df_mul(L[0], Y[3]), df_mul(L[1], Y[4])), df_mul(L[2], Y[5]));
-  const df2 pp = df_add(df_add(df_mul(Y[3], Y[3]), df_mul(Y[4], Y[4])), df_mul(Y[5], Y[5]));
-  const df2 A = df_sub(pp, df_mul(f, df_mul(kap, kap)));
-  const df2 B = df_mulf(df_mul(df_mul(f, PT), kap), 2.f);
-  const df2 C = df_neg(df_mul(df_add(dfq(1.f), f), df_mul(PT, PT)));
-  const df2 disc = df_sub(df_mul(B, B), df_mulf(df_mul(A, C), 4.f));
+  const df2 pp = dot3(Y[3], Y[3], Y[4], Y[4], Y[5], Y[5]);
+  const df2 A = fma1(neg(f), mul(kap, kap), pp);
+  const df2 B = scale(mul(mul(f, pt), kap), 2.f);
+  const df2 C = neg(mul(addf(f, 1.f), mul(pt, pt)));
+  const df2 disc = fma1(scale(A, -4.f), C, mul(B, B));
   if (!(A.hi > 0.f) || !(disc.hi >= 0.f)) return;
-  const df2 lam = df_mul(df_sub(df_sqrt(disc), B), df_rcp(df_mulf(A, 2.f)));
+  const df2 lam = mul(sub(sqrt_(disc), B), rcp(scale(A, 2.f)));
   if (!(lam.hi > 0.9f && lam.hi < 1.1f)) return;
 #pragma unroll
   for (int i = 3; i < 6; ++i) {
-    const df2 v = df_mul(Y[i], lam);
+    const df2 v = mul(Y[i], lam);
     y[i] = v.hi;
     lo[i] = v.lo;
-  }
-}
-
-template <int KERR>
-__device__ __forceinline__ void renorm_fp64(float* y, float* lo, float pt, double M, double a) {
-  double yd[6];
-#pragma unroll
-  for (int k = 0; k < 6; ++k) yd[k] = (double)y[k] + (double)lo[k];
-  null_renorm<KERR>(yd, (double)pt, M, a);
-#pragma unroll
-  for (int k = 3; k < 6; ++k) {
-    const float hi = (float)yd[k];
-    y[k] = hi;
-    lo[k] = (float)(yd[k] - (double)hi);
   }
 }
 
@@ -1548,9 +1302,7 @@ __device__ __forceinline__ bool step_ray(const TraceParams& p, RayState<typename
     st.k1_valid = true;
   } else if (fp64_step) {
     if constexpr (PREC == ST_PREC_FP32_GUARDED) {
-      // the guard step: FP64, or double-float on the FP32 pipe (counted alike)
-      if (p.guard_df) guard_step_df<KERR>(y, st.lo, st.pt, p, h);
-      else guard_step_fp64<KERR>(y, st.lo, st.pt, p.M, p.a, h);
+      guard_step<KERR>(y, st.lo, st.pt, p, h);
       ++st.fp64_steps;
     }
   } else {
@@ -1572,10 +1324,7 @@ __device__ __forceinline__ bool step_ray(const TraceParams& p, RayState<typename
   }
   ++st.steps;
   if constexpr (PREC == ST_PREC_FP32_GUARDED) {
-    if (p.renorm_every > 0 && (st.steps % p.renorm_every) == 0) {
-      if (p.guard_df) renorm_df<KERR>(y, st.lo, st.pt, p);
-      else renorm_fp64<KERR>(y, st.lo, st.pt, p.M, p.a);
-    }
+    if (p.renorm_every > 0 && (st.steps % p.renorm_every) == 0) null_renorm<KERR>(y, st.lo, st.pt, p);
   }
   if (!(y[0] == y[0]) || !(y[2] == y[2]) || !(y[3] == y[3])) { st.flags |= ST_RAY_CAPTURED; return true; }
 
