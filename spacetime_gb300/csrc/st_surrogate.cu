@@ -30,10 +30,11 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cmath>
 #include <cstddef>
 #include <cstdlib>
-#include <cmath>
 #include <cstring>
+#include <type_traits>
 #include <new>
 #include <vector>
 
@@ -120,47 +121,42 @@ __global__ void l4_fwd(const __nv_bfloat16* __restrict__ H3, const float* __rest
 // o2 is unused and carries no gradient.
 // loss_acc[0..3] += (total, direction MSE, radius MSE, g MSE) / B
 constexpr float WR = 1.0f, WG = 1.0f;
+__device__ __forceinline__ void row_loss(const float* o, const float* __restrict__ t, float* g, float* l) {
+  const float md = t[5], mc = t[6];
+  const float s = fminf(fmaxf(o[5], -30.f), 12.f);
+  const float es = __expf(-s);
+  float e2 = 0.f;
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    const float e = o[k] - t[k];
+    e2 += e * e;
+    g[k] = md * e * es;
+  }
+  g[2] = 0.f;
+  g[5] = (o[5] > -30.f && o[5] < 12.f) ? md * (-0.5f * e2 * es + 1.f) : 0.f;
+  const float er = o[3] - t[3], eg = o[4] - t[4];
+  g[3] = 2.f * WR * er;
+  g[4] = 2.f * WG * mc * eg;
+  l[1] = md * e2;
+  l[2] = er * er;
+  l[3] = mc * eg * eg;
+  l[0] = md * (0.5f * e2 * es + s) + WR * l[2] + WG * l[3];
+}
 __global__ void loss_grad(const float* __restrict__ out, const float* __restrict__ T, float* dout, float* loss_acc,
                           int B, float inv_batch) {
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  float l_tot = 0.f, l_dir = 0.f, l_r = 0.f, l_g = 0.f;
+  float l[4] = {0.f, 0.f, 0.f, 0.f};
   if (b < B) {
-    const float* o = out + (size_t)b * NOUT;
-    const float* t = T + (size_t)b * NT;
-    const float md = t[5], mc = t[6];
-    const float s = fminf(fmaxf(o[5], -30.f), 12.f);
-    const float es = __expf(-s);
-    float e2 = 0.f, g[NOUT];
-#pragma unroll
-    for (int k = 0; k < 2; ++k) {
-      const float e = o[k] - t[k];
-      e2 += e * e;
-      g[k] = md * e * es;
-    }
-    g[2] = 0.f;
-    g[5] = (o[5] > -30.f && o[5] < 12.f) ? md * (-0.5f * e2 * es + 1.f) : 0.f;
-    const float er = o[3] - t[3], eg = o[4] - t[4];
-    g[3] = 2.f * WR * er;
-    g[4] = 2.f * WG * mc * eg;
+    float g[NOUT];
+    row_loss(out + (size_t)b * NOUT, T + (size_t)b * NT, g, l);
 #pragma unroll
     for (int k = 0; k < NOUT; ++k) dout[(size_t)b * NOUT + k] = g[k] * inv_batch;
-    l_dir = md * e2;
-    l_r = er * er;
-    l_g = mc * eg * eg;
-    l_tot = md * (0.5f * e2 * es + s) + WR * l_r + WG * l_g;
   }
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    l_tot += __shfl_xor_sync(0xffffffffu, l_tot, o);
-    l_dir += __shfl_xor_sync(0xffffffffu, l_dir, o);
-    l_r += __shfl_xor_sync(0xffffffffu, l_r, o);
-    l_g += __shfl_xor_sync(0xffffffffu, l_g, o);
-  }
-  if ((threadIdx.x & 31) == 0) {
-    atomicAdd(loss_acc + 0, l_tot * inv_batch);
-    atomicAdd(loss_acc + 1, l_dir * inv_batch);
-    atomicAdd(loss_acc + 2, l_r * inv_batch);
-    atomicAdd(loss_acc + 3, l_g * inv_batch);
+  for (int k = 0; k < 4; ++k) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) l[k] += __shfl_xor_sync(0xffffffffu, l[k], o);
+    if ((threadIdx.x & 31) == 0) atomicAdd(loss_acc + k, l[k] * inv_batch);
   }
 }
 
@@ -1606,6 +1602,14 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
   }
 }
 
+}  // namespace sur
+}  // namespace st
+
+#include "st_train.cuh"
+
+namespace st {
+namespace sur {
+
 // Grid of the persistent network kernel: one CTA per SM, at most one per tile.
 inline int tc_grid(int ntiles) {
   int dev = 0, nsm = 0;
@@ -1624,16 +1628,18 @@ inline int tc_grid(int ntiles) {
 
 extern "C" void st_surrogate_destroy(st_surrogate* s);
 
+constexpr int THIST = 1024;  // training steps whose losses wait on the device
+
 struct st_surrogate {
   int device = 0;
   cudaStream_t stream = nullptr;
   float *P = nullptr, *G = nullptr, *Mm = nullptr, *Vv = nullptr;
   __nv_bfloat16* Wb[3] = {nullptr, nullptr, nullptr};
-  __nv_bfloat16* Wt[3] = {nullptr, nullptr, nullptr};  // W^T (bf16) for the tcgen05 input-gradient GEMM
-  // [256][cap] transposes for the weight gradient: H_0..H_2 (written by the
-  // forward epilogues) and dZ (ping-pong, written by the input-gradient epilogues)
-  __nv_bfloat16* HT[3] = {nullptr, nullptr, nullptr};
-  __nv_bfloat16* dZT[2] = {nullptr, nullptr};
+  // training: hidden weights and their transposes as swizzled images, the tiles
+  // between its kernels, their partial sums, THIST steps' losses
+  unsigned char *WF = nullptr, *WT = nullptr, *tH = nullptr, *tD = nullptr;
+  float *tZ = nullptr, *tpart = nullptr, *tpw = nullptr, *thist = nullptr;
+  int ttiles = 0;
   unsigned* d_queue = nullptr;  // head of the label kernel's sample queue, and label_order's two histograms
   uint32_t* d_order = nullptr;  // label_order's rows
   int order_cap = 0;
@@ -1678,8 +1684,6 @@ int ensure_work(st_surrogate* s, int rows) {
   cudaFree(s->X);
   for (int l = 0; l < 4; ++l) { cudaFree(s->Z[l]); cudaFree(s->H[l]); }
   cudaFree(s->dZa); cudaFree(s->dZb); cudaFree(s->out); cudaFree(s->dout); cudaFree(s->T);
-  for (int l = 0; l < 3; ++l) { cudaFree(s->HT[l]); s->HT[l] = nullptr; }
-  for (int l = 0; l < 2; ++l) { cudaFree(s->dZT[l]); s->dZT[l] = nullptr; }
   cudaFree(s->part);
   s->part = nullptr;
   s->cap = 0;
@@ -1694,28 +1698,22 @@ int ensure_work(st_surrogate* s, int rows) {
   if (cudaMalloc(&s->out, R * NOUT * 4) != cudaSuccess || cudaMalloc(&s->dout, R * NOUT * 4) != cudaSuccess ||
       cudaMalloc(&s->T, R * NT * 4) != cudaSuccess)
     return ST_ENOMEM;
-  for (int l = 0; l < 3; ++l)
-    if (cudaMalloc(&s->HT[l], R * NH * 2) != cudaSuccess) return ST_ENOMEM;
-  for (int l = 0; l < 2; ++l)
-    if (cudaMalloc(&s->dZT[l], R * NH * 2) != cudaSuccess) return ST_ENOMEM;
   if (cudaMalloc(&s->part, (R / RED_ROWS + 1) * (size_t)L0_PART * 4) != cudaSuccess) return ST_ENOMEM;
   s->cap = rows;
   return ST_OK;
 }
 
-// The training kernels' bf16 copies of the hidden weights (and W^T), after
-// every parameter update.
+// The bf16 copies of the hidden weights that the layer-by-layer kernels read.
 int sync_bf16(st_surrogate* s) {
   for (int l = 0; l < 3; ++l) {
     to_bf16<<<(NH * NH + 255) / 256, 256, 0, s->stream>>>(s->P + OWH[l], s->Wb[l], NH * NH);
-    SC(cudaGetLastError());
-    st::tcg::transpose_bf16<<<dim3(NH / 32, NH / 32), 256, 0, s->stream>>>(s->Wb[l], s->Wt[l], NH, NH);
     SC(cudaGetLastError());
   }
   return ST_OK;
 }
 
-// The tensor-core network kernel's weight images and packed biases: once the
+// The weight images of the tensor-core network kernel and of training, and the
+// packed biases: once the
 // parameters are final (creation, st_surrogate_set_params, the end of
 // st_surrogate_train), not after every training step.
 int sync_tc_images(st_surrogate* s) {
@@ -1723,20 +1721,22 @@ int sync_tc_images(st_surrogate* s) {
   SC(cudaGetLastError());
   pack_small<<<(TC_SMALL_BYTES / 4 + 255) / 256, 256, 0, s->stream>>>(s->P, s->Psmall);
   SC(cudaGetLastError());
+  pack_train<<<3 * NH * NH / 256, 256, 0, s->stream>>>(s->P, s->WF, s->WT);
+  SC(cudaGetLastError());
   return ST_OK;
 }
 
-// The hidden-layer GEMMs of training and of st_surrogate_forward run on
-// tcgen05 (st_tcgemm.cuh) unless SPACETIME_GB300_TRAIN_MMA=sync selects the
+// The hidden-layer GEMMs of training (st_train.cuh) and of st_surrogate_forward
+// (st_tcgemm.cuh) run on tcgen05 unless SPACETIME_GB300_TRAIN_MMA=sync selects the
 // mma.sync kernels (st_mlp.cuh), the same computation on the warp-level path.
 bool train_on_tcgen05() {
   const char* e = std::getenv("SPACETIME_GB300_TRAIN_MMA");
   return !(e && std::strcmp(e, "sync") == 0);
 }
 
-// C[M][256] = A[M][K] B[256][K]^T on tcgen05, K split over gridDim.z.
+// C[M][256] = A[M][K] B[256][K]^T on tcgen05.
 template <class Epi>
-int gemm_tc(const __nv_bfloat16* A, int lda, const __nv_bfloat16* B, int ldb, int M, int K, int splits, Epi epi,
+int gemm_tc(const __nv_bfloat16* A, int lda, const __nv_bfloat16* B, int ldb, int M, int K, Epi epi,
             int* status, cudaStream_t st) {
   static bool attr = false;  // one instantiation per epilogue
   if (!attr) {
@@ -1744,7 +1744,7 @@ int gemm_tc(const __nv_bfloat16* A, int lda, const __nv_bfloat16* B, int ldb, in
                             (int)st::tcg::SMEM));
     attr = true;
   }
-  st::tcg::gemm_tc_kernel<Epi><<<dim3(1, M / st::tcg::TILE_M, splits), st::tcg::THREADS, st::tcg::SMEM, st>>>(
+  st::tcg::gemm_tc_kernel<Epi><<<dim3(1, M / st::tcg::TILE_M), st::tcg::THREADS, st::tcg::SMEM, st>>>(
       A, lda, B, ldb, K, epi, status);
   SC(cudaGetLastError());
   return ST_OK;
@@ -1755,18 +1755,11 @@ int forward(st_surrogate* s, const float* X, int B, bool keep_z, cudaStream_t st
   l0_fwd<<<(B + L0_ROWS - 1) / L0_ROWS, NH, 0, st>>>(X, s->P, keep_z ? s->Z[0] : nullptr, s->H[0], B);
   SC(cudaGetLastError());
   const bool tc5 = train_on_tcgen05();
-  if (tc5 && keep_z) {
-    // training: H_0^T for the first layer's weight gradient (the GEMM
-    // epilogues write H_1^T and H_2^T themselves)
-    st::tcg::transpose_bf16<<<dim3(NH / 32, B / 32), 256, 0, st>>>(s->H[0], s->HT[0], B, NH);
-    SC(cudaGetLastError());
-  }
   for (int l = 1; l <= 3; ++l) {
     EpiHidden e{s->P + OBH[l - 1], keep_z ? s->Z[l] : nullptr, s->H[l], NH};
     if (tc5) {
       // Z = H W^T: A = H [B][256], B = W [256 out][256 in], both K-major
-      if (keep_z && l < 3) { e.T = s->HT[l]; e.ldt = B; }
-      const int rc = gemm_tc(s->H[l - 1], NH, s->Wb[l - 1], NH, B, NH, 1, e, s->d_status, st);
+      const int rc = gemm_tc(s->H[l - 1], NH, s->Wb[l - 1], NH, B, NH, e, s->d_status, st);
       if (rc != ST_OK) return rc;
       continue;
     }
@@ -1791,7 +1784,8 @@ int l0_backward(st_surrogate* s, const __nv_bfloat16* dZ0, const float* X, int B
   return ST_OK;
 }
 
-// backward from s->dout (already scaled by 1/B); accumulates into s->G
+// backward from s->dout (already scaled by 1/B) layer by layer on mma.sync;
+// accumulates into s->G
 int backward(st_surrogate* s, const float* X, int B) {
   cudaStream_t st = s->stream;
   SC(cudaMemsetAsync(s->G, 0, NPARAM * 4, st));
@@ -1806,31 +1800,6 @@ int backward(st_surrogate* s, const float* X, int B) {
   __nv_bfloat16* dZ = s->dZa;
   __nv_bfloat16* dZn = s->dZb;
   const int splits = std::max(1, std::min(64, B / 1024));
-  if (train_on_tcgen05()) {
-    // both weight-gradient operands K-major over the batch: dZ^T and H^T
-    // (written transposed by the forward and input-gradient epilogues; dZ_3,
-    // from the FP32 output layer, transposed here); K = 1024 per split keeps
-    // the atomics few and the pipeline full
-    st::tcg::transpose_bf16<<<dim3(NH / 32, B / 32), 256, 0, st>>>(dZ, s->dZT[0], B, NH);
-    SC(cudaGetLastError());
-    int cur = 0;
-    for (int l = 3; l >= 1; --l) {
-      // dW_l[o][i] = sum_b dZ[b][o] H_{l-1}[b][i]: A = dZ^T [256][B], B = H^T [256][B]
-      EpiAccum ea{s->G + OWH[l - 1], NH};
-      int rc = gemm_tc(s->dZT[cur], B, s->HT[l - 1], B, NH, B, splits, ea, s->d_status, st);
-      if (rc != ST_OK) return rc;
-      colsum_bf16<<<nred, NH, 0, st>>>(dZ, s->G, OBH[l - 1], B);
-      SC(cudaGetLastError());
-      // dZ_{l-1}[b][i] = (sum_o dZ[b][o] W[o][i]) silu'(Z_{l-1}): A = dZ [B][256], B = W^T [256 in][256 out]
-      EpiBackDX eb{s->Z[l - 1], dZn, NH};
-      if (l > 1) { eb.T = s->dZT[cur ^ 1]; eb.ldt = B; }
-      rc = gemm_tc(dZ, NH, s->Wt[l - 1], NH, B, NH, 1, eb, s->d_status, st);
-      if (rc != ST_OK) return rc;
-      std::swap(dZ, dZn);
-      cur ^= 1;
-    }
-    return l0_backward(s, dZ, X, B, nred);
-  }
   for (int l = 3; l >= 1; --l) {
     // dW_l = dZ_l^T H_{l-1}
     EpiAccum ea{s->G + OWH[l - 1], NH};
@@ -1873,6 +1842,44 @@ int label_order(st_surrogate* s, LabelParams* lp) {
   SC(cudaGetLastError());
   lp->order = s->d_order;
   lp->sorted = m;
+  return ST_OK;
+}
+
+// Buffers of the training kernels for ntiles 128-row tiles.
+int ensure_train(st_surrogate* s, int ntiles) {
+  if (ntiles <= s->ttiles) return ST_OK;
+  cudaFree(s->tH); cudaFree(s->tD); cudaFree(s->tZ); cudaFree(s->tpart); cudaFree(s->tpw);
+  s->tH = s->tD = nullptr;
+  s->tZ = s->tpart = s->tpw = nullptr;
+  s->ttiles = 0;
+  const size_t nt = ntiles, grid = tc_grid(ntiles);
+  if (cudaMalloc(&s->tH, 3 * nt * TR_IMG) != cudaSuccess || cudaMalloc(&s->tD, 3 * nt * TR_IMG) != cudaSuccess ||
+      cudaMalloc(&s->tZ, grid * 2 * NH * TC_ROWS * sizeof(float)) != cudaSuccess ||
+      cudaMalloc(&s->tpart, grid * TR_ROW * sizeof(float)) != cudaSuccess ||
+      cudaMalloc(&s->tpw, (size_t)TR_SPLITS * 3 * NH * NH * sizeof(float)) != cudaSuccess)
+    return ST_ENOMEM;
+  SC(cudaFuncSetAttribute(train_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TR_SMEM));
+  SC(cudaFuncSetAttribute(train_dw_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DW_SMEM));
+  // all three kernels of a step on one split of L1, so no SM changes it between them
+  SC(cudaFuncSetAttribute(train_update_kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
+                          cudaSharedmemCarveoutMaxShared));
+  s->ttiles = ntiles;
+  return ST_OK;
+}
+
+// Loss sums (added to loss[4]) and gradient of B padded rows, n of which count,
+// into G or, where G is null, an AdamW step.
+int train_pass(st_surrogate* s, const float* X, const float* T, int B, int n, float* loss, float* G,
+               const AdamParams& a) {
+  const int nt = B / (int)TC_ROWS, grid = tc_grid(nt), splits = std::min(TR_SPLITS, nt);
+  const TrainParams tp{s->P, s->WF, s->WT, X, T, n, nt, 1.0f / n, s->tH, s->tD, s->tZ, s->tpart, loss, s->d_status};
+  train_tile_kernel<<<grid, TR_THREADS, TR_SMEM, s->stream>>>(tp);
+  SC(cudaGetLastError());
+  train_dw_kernel<<<dim3(splits, 2, 3), 256, DW_SMEM, s->stream>>>(s->tH, s->tD, nt, s->tpw, s->d_status);
+  SC(cudaGetLastError());
+  train_update_kernel<<<UPD_HIDDEN + UPD_EDGE, 256, 0, s->stream>>>(s->tpw, splits, s->tpart, grid, G, a, s->WF,
+                                                                    s->WT);
+  SC(cudaGetLastError());
   return ST_OK;
 }
 
@@ -1946,11 +1953,13 @@ int st_surrogate_create(st_surrogate** out, int device, unsigned long long seed)
   if (cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking) != cudaSuccess) return fail(ST_ECUDA);
   if (cudaMalloc(&s->P, NPARAM * 4) != cudaSuccess || cudaMalloc(&s->G, NPARAM * 4) != cudaSuccess ||
       cudaMalloc(&s->Mm, NPARAM * 4) != cudaSuccess || cudaMalloc(&s->Vv, NPARAM * 4) != cudaSuccess ||
-      cudaMalloc(&s->loss, 16 * 4) != cudaSuccess)
+      cudaMalloc(&s->loss, 16 * 4) != cudaSuccess ||
+      cudaMalloc(&s->thist, 4 * THIST * sizeof(float)) != cudaSuccess)
     return fail(ST_ENOMEM);
   for (int l = 0; l < 3; ++l)
-    if (cudaMalloc(&s->Wb[l], NH * NH * 2) != cudaSuccess || cudaMalloc(&s->Wt[l], NH * NH * 2) != cudaSuccess)
-      return fail(ST_ENOMEM);
+    if (cudaMalloc(&s->Wb[l], NH * NH * 2) != cudaSuccess) return fail(ST_ENOMEM);
+  if (cudaMalloc(&s->WF, 3 * TC_B_BYTES) != cudaSuccess || cudaMalloc(&s->WT, 3 * TC_B_BYTES) != cudaSuccess)
+    return fail(ST_ENOMEM);
   if (cudaMalloc(&s->d_status, sizeof(int)) != cudaSuccess || cudaMemset(s->d_status, 0, sizeof(int)) != cudaSuccess)
     return fail(ST_ENOMEM);
   if (cudaMalloc(&s->d_queue, (1 + 2 * ORDER_BUCKETS) * sizeof(unsigned)) != cudaSuccess) return fail(ST_ENOMEM);
@@ -1994,12 +2003,12 @@ void st_surrogate_destroy(st_surrogate* s) {
   cudaSetDevice(s->device);
   if (s->stream) cudaStreamSynchronize(s->stream);
   cudaFree(s->P); cudaFree(s->G); cudaFree(s->Mm); cudaFree(s->Vv); cudaFree(s->loss);
-  for (int l = 0; l < 3; ++l) { cudaFree(s->Wb[l]); cudaFree(s->Wt[l]); }
+  for (int l = 0; l < 3; ++l) cudaFree(s->Wb[l]);
+  cudaFree(s->WF); cudaFree(s->WT); cudaFree(s->tH); cudaFree(s->tD); cudaFree(s->tZ); cudaFree(s->tpart);
+  cudaFree(s->tpw); cudaFree(s->thist);
   cudaFree(s->d_status);
   cudaFree(s->d_queue);
   cudaFree(s->d_order);
-  for (int l = 0; l < 3; ++l) cudaFree(s->HT[l]);
-  for (int l = 0; l < 2; ++l) cudaFree(s->dZT[l]);
   cudaFree(s->part);
   cudaFree(s->Wsw);
   cudaFree(s->Psmall);
@@ -2084,13 +2093,18 @@ int st_surrogate_loss_grad(st_surrogate* s, const float* X, const float* T, int 
   SC(cudaMemsetAsync(s->T, 0, (size_t)B * NT * 4, st));
   SC(cudaMemcpyAsync(s->X, X, (size_t)n * NIN * 4, cudaMemcpyHostToDevice, st));
   SC(cudaMemcpyAsync(s->T, T, (size_t)n * NT * 4, cudaMemcpyHostToDevice, st));
-  if ((rc = forward(s, s->X, B, true, s->stream)) != ST_OK) return rc;
   SC(cudaMemsetAsync(s->loss, 0, 16 * 4, st));
-  loss_grad<<<(B + 255) / 256, 256, 0, st>>>(s->out, s->T, s->dout, s->loss, n, 1.0f / n);
-  SC(cudaGetLastError());
-  // padding rows carry no gradient
-  if (B > n) SC(cudaMemsetAsync(s->dout + (size_t)n * NOUT, 0, (size_t)(B - n) * NOUT * 4, st));
-  if ((rc = backward(s, s->X, B)) != ST_OK) return rc;
+  if (train_on_tcgen05()) {
+    if ((rc = ensure_train(s, B / (int)TC_ROWS)) != ST_OK) return rc;
+    if ((rc = train_pass(s, s->X, s->T, B, n, s->loss, s->G, AdamParams{})) != ST_OK) return rc;
+  } else {
+    if ((rc = forward(s, s->X, B, true, s->stream)) != ST_OK) return rc;
+    loss_grad<<<(B + 255) / 256, 256, 0, st>>>(s->out, s->T, s->dout, s->loss, n, 1.0f / n);
+    SC(cudaGetLastError());
+    // padding rows carry no gradient
+    if (B > n) SC(cudaMemsetAsync(s->dout + (size_t)n * NOUT, 0, (size_t)(B - n) * NOUT * 4, st));
+    if ((rc = backward(s, s->X, B)) != ST_OK) return rc;
+  }
   if (loss4) SC(cudaMemcpyAsync(loss4, s->loss, 4 * 4, cudaMemcpyDeviceToHost, st));
   if (grad) SC(cudaMemcpyAsync(grad, s->G, NPARAM * 4, cudaMemcpyDeviceToHost, st));
   SC(cudaStreamSynchronize(st));
@@ -2142,34 +2156,51 @@ int st_surrogate_train(st_surrogate* s, int steps, int batch, float lr, float we
   if (!s || steps <= 0 || batch < 128 || batch % 128 != 0) return ST_EINVAL;
   if (s->ndata < batch) return ST_ESTATE;
   if (cudaSetDevice(s->device) != cudaSuccess) return ST_ECUDA;
-  int rc = ensure_work(s, batch);
+  const bool tc5 = train_on_tcgen05();
+  int rc = tc5 ? ensure_train(s, batch / (int)TC_ROWS) : ensure_work(s, batch);
   if (rc != ST_OK) return rc;
   cudaStream_t st = s->stream;
   const long long nb = s->ndata / batch;
-  std::vector<float> lh(steps > 0 ? steps : 1);
+  // the loss sums of THIST steps stay on the device and come back together
+  std::vector<float> lh(4 * THIST);
+  const auto fetch = [&](int k0, int k1) {
+    if (!loss_hist || k1 <= k0) return ST_OK;
+    SC(cudaMemcpyAsync(lh.data(), s->thist, 4 * sizeof(float) * (k1 - k0), cudaMemcpyDeviceToHost, st));
+    SC(cudaStreamSynchronize(st));
+    for (int k = k0; k < k1; ++k) loss_hist[k] = lh[4 * (size_t)(k - k0)];
+    return ST_OK;
+  };
   for (int k = 0; k < steps; ++k) {
+    if (k % THIST == 0) {
+      if (k && (rc = fetch(k - THIST, k)) != ST_OK) return rc;
+      SC(cudaMemsetAsync(s->thist, 0, 4 * THIST * sizeof(float), st));
+    }
     const long long bi = (s->step * 7919LL) % nb;  // stride through the batches
     const float* X = s->DX + bi * batch * NIN;
     const float* T = s->DT + bi * batch * NT;
-    if ((rc = forward(s, X, batch, true, s->stream)) != ST_OK) return rc;
-    SC(cudaMemsetAsync(s->loss, 0, 16 * 4, st));
-    loss_grad<<<(batch + 255) / 256, 256, 0, st>>>(s->out, T, s->dout, s->loss, batch, 1.0f / batch);
-    SC(cudaGetLastError());
-    if ((rc = backward(s, X, batch)) != ST_OK) return rc;
+    float* loss = s->thist + 4 * (k % THIST);
     ++s->step;
     const float b1 = 0.9f, b2 = 0.999f;
     const float bc1 = 1.f - std::pow(b1, (float)s->step), bc2 = 1.f - std::pow(b2, (float)s->step);
+    if (tc5) {
+      const AdamParams a{s->P, s->Mm, s->Vv, lr, b1, b2, 1e-8f, weight_decay, bc1, bc2};
+      if ((rc = train_pass(s, X, T, batch, batch, loss, nullptr, a)) != ST_OK) return rc;
+      continue;
+    }
+    if ((rc = forward(s, X, batch, true, s->stream)) != ST_OK) return rc;
+    loss_grad<<<(batch + 255) / 256, 256, 0, st>>>(s->out, T, s->dout, loss, batch, 1.0f / batch);
+    SC(cudaGetLastError());
+    if ((rc = backward(s, X, batch)) != ST_OK) return rc;
     adamw<<<(unsigned)((NPARAM + 255) / 256), 256, 0, st>>>(s->P, s->G, s->Mm, s->Vv, NPARAM, lr, b1, b2, 1e-8f,
                                                            weight_decay, bc1, bc2);
     SC(cudaGetLastError());
     if ((rc = sync_bf16(s)) != ST_OK) return rc;
-    if (loss_hist) SC(cudaMemcpyAsync(&lh[k], s->loss, 4, cudaMemcpyDeviceToHost, st));
   }
+  if (tc5 && (rc = sync_bf16(s)) != ST_OK) return rc;
   if ((rc = sync_tc_images(s)) != ST_OK) return rc;
+  if ((rc = fetch((steps - 1) / THIST * THIST, steps)) != ST_OK) return rc;
   SC(cudaStreamSynchronize(st));
-  if ((rc = gemm_status(s)) != ST_OK) return rc;
-  if (loss_hist) std::memcpy(loss_hist, lh.data(), steps * sizeof(float));
-  return ST_OK;
+  return gemm_status(s);
 }
 
 }  // extern "C"

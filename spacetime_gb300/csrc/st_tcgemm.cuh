@@ -1,6 +1,7 @@
 // st_tcgemm.cuh -- BF16 GEMM on the 5th-generation tensor cores for the
-// surrogate's training passes: C[M][256] = A[M][K] . B[256][K]^T, both
-// operands K-major bf16, FP32 accumulation in tensor memory, fused epilogue.
+// surrogate's forward pass (training has its own, st_train.cuh): C[M][256] =
+// A[M][K] . B[256][K]^T, both operands K-major bf16, FP32 accumulation in
+// tensor memory, fused epilogue.
 //
 // One CTA computes a 128 x 256 tile (M = 128 rows of A, all 256 rows of B)
 // with one 128-lane x 256-column TMEM accumulator.  K runs in blocks of 64
@@ -9,8 +10,7 @@
 // st_tc.cuh), four stages deep (a K = 256 layer's whole operands in flight
 // at once); one thread issues the block's four tcgen05.mma (M = 128, N = 256,
 // K = 16) and commits them to an mbarrier, which tells the copy of the block
-// four ahead that the stage is free.  gridDim.z splits K (the epilogue then
-// accumulates, e.g. with atomics).
+// four ahead that the stage is free.
 //
 // Every mbarrier wait is bounded.  A wait that runs out sets *status, the
 // issuing thread waits again (bounded) for its last committed MMAs, and the
@@ -55,14 +55,10 @@ __device__ __forceinline__ void load_block(unsigned char* As, unsigned char* Bs,
   }
 }
 
-// Epilogue contract: epi.store(m, n, v, a) receives C[m][n] and a = epi.pre(m, n),
-// the epilogue's own operand at (m, n) (read for a whole block before any of
-// its stores), and returns its output value; with epi.T set that value is also
-// written transposed, T[n * epi.ldt + m] (bf16).  Each warp moves a 32 x 32
-// block of the accumulator (its TMEM lanes = rows, 32 columns) through shared
-// memory, so the epilogue runs a row at a time across the warp's lanes and its
-// loads, stores and atomics are coalesced along n, and the transposed copy a
-// column at a time, coalesced along m.
+// Epilogue contract: epi.store(m, n, v) receives v = C[m][n].  Each warp moves
+// a 32 x 32 block of the accumulator (its TMEM lanes = rows, 32 columns)
+// through shared memory, so the epilogue runs a row at a time across the
+// warp's lanes and its loads and stores are coalesced along n.
 template <class Epi>
 __global__ void __launch_bounds__(THREADS, 1)
     gemm_tc_kernel(const __nv_bfloat16* __restrict__ A, int lda, const __nv_bfloat16* __restrict__ B, int ldb, int K,
@@ -77,11 +73,7 @@ __global__ void __launch_bounds__(THREADS, 1)
   int* fail = reinterpret_cast<int*>(bar + 2);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int m0 = blockIdx.y * TILE_M;
-  // split-K range of this CTA, in whole K-blocks
-  const int nkb_all = K / KB;
-  const int per = (nkb_all + (int)gridDim.z - 1) / (int)gridDim.z;
-  const int kb0 = blockIdx.z * per;
-  const int nkb = min(nkb_all - kb0, per);
+  const int nkb = K / KB;
   if (nkb <= 0) return;  // uniform over the CTA: nothing allocated yet
   if (tid == 0) {
     tc::mbar_init(bar, 1);
@@ -97,7 +89,7 @@ __global__ void __launch_bounds__(THREADS, 1)
   // prologue: blocks 0 .. STAGES-2
 #pragma unroll
   for (int s = 0; s < STAGES - 1; ++s) {
-    if (s < nkb) load_block(Ast + s * A_STAGE, Bst + s * B_STAGE, A, lda, B, ldb, m0, (kb0 + s) * KB, tid);
+    if (s < nkb) load_block(Ast + s * A_STAGE, Bst + s * B_STAGE, A, lda, B, ldb, m0, s * KB, tid);
     cp_commit();
   }
   for (int kb = 0; kb < nkb; ++kb) {
@@ -110,7 +102,7 @@ __global__ void __launch_bounds__(THREADS, 1)
     const int ahead = kb + STAGES - 1;
     if (ahead < nkb) {
       const int sa = ahead % STAGES;
-      load_block(Ast + sa * A_STAGE, Bst + sa * B_STAGE, A, lda, B, ldb, m0, (kb0 + ahead) * KB, tid);
+      load_block(Ast + sa * A_STAGE, Bst + sa * B_STAGE, A, lda, B, ldb, m0, ahead * KB, tid);
     }
     cp_commit();
     cp_wait<STAGES - 1>();   // block kb's copies have landed
@@ -148,24 +140,14 @@ __global__ void __launch_bounds__(THREADS, 1)
     for (int c = 0; c < 4; ++c) {
       const int col0 = (int)ch * 128 + c * 32;
       const int mq = m0 + (int)(q * 32);
-      float pre[32];
-#pragma unroll
-      for (int r = 0; r < 32; ++r) pre[r] = epi.pre(mq + r, col0 + lane);
       float v[32];
       tc::tmem_ld32(tmem + ((q * 32u) << 16) + (uint32_t)col0, v);
 #pragma unroll
       for (int e = 0; e < 32; ++e) tile[lane * 33 + e] = v[e];
       __syncwarp();
 #pragma unroll
-      for (int r = 0; r < 32; ++r)
-        tile[r * 33 + lane] = epi.store(mq + r, col0 + lane, tile[r * 33 + lane], pre[r]);
+      for (int r = 0; r < 32; ++r) epi.store(mq + r, col0 + lane, tile[r * 33 + lane]);
       __syncwarp();
-      if (epi.T) {
-#pragma unroll 8
-        for (int c = 0; c < 32; ++c)
-          epi.T[(size_t)(col0 + c) * epi.ldt + mq + lane] = __float2bfloat16_rn(tile[lane * 33 + c]);
-        __syncwarp();
-      }
     }
   }
   tc::fence_before_sync();
@@ -175,19 +157,6 @@ __global__ void __launch_bounds__(THREADS, 1)
     tc::tmem_dealloc(tmem, 256);
   }
   if (failed && tid == 0 && status) atomicExch(status, 1);
-}
-
-// dst[c][r] = src[r][c] for a rows x cols bf16 matrix (both multiples of 32).
-__global__ void __launch_bounds__(256) transpose_bf16(const __nv_bfloat16* __restrict__ src,
-                                                      __nv_bfloat16* __restrict__ dst, int rows, int cols) {
-  __shared__ __nv_bfloat16 t[32][34];
-  const int c0 = blockIdx.x * 32, r0 = blockIdx.y * 32;
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-#pragma unroll
-  for (int i = 0; i < 32; i += 8) t[ty + i][tx] = src[(size_t)(r0 + ty + i) * cols + c0 + tx];
-  __syncthreads();
-#pragma unroll
-  for (int i = 0; i < 32; i += 8) dst[(size_t)(c0 + ty + i) * rows + r0 + tx] = t[tx][ty + i];
 }
 
 }  // namespace tcg
