@@ -479,8 +479,8 @@ def fluid_variant(ctx_cls, device: int, steps: int = 200) -> dict:
     """The live fluid disc (DiscFluidSim / step_sim!, dt 0.08, jacobi 8) on two
     grids: config 1's gas grid (256 x 64 x 32, ISCO to 25 M) and the
     reference's default DiscVolume grid (192 x 256 x 48, 3-20 M).  Device time
-    per step through the CUDA graph and as plain stream launches (4 kernels a
-    step), and the oracle's single-thread CPU time per step."""
+    per step of one call of `steps` steps and of as many calls of one step, and
+    the oracle's single-thread CPU time per step."""
     import time
 
     import numpy as np
@@ -495,23 +495,22 @@ def fluid_variant(ctx_cls, device: int, steps: int = 200) -> dict:
              AccretionDisc(3.0, 20.0, Blackbody(wb_temperature=10000.0), 0.8))):
         ctx = ctx_cls(workloads.sky(256, 128), disc=disc, volume=vol, device=device)
         sim = DiscFluidSim(ctx, vol, disc)
-        sim.step(dt=0.08, nsteps=20, graph=True, timed=True)          # warm-up (and graph build)
-        ms_graph = sim.step(dt=0.08, nsteps=steps, graph=True, timed=True) / steps
-        sim.step(dt=0.08, nsteps=20, graph=False, timed=True)
-        ms_plain = sim.step(dt=0.08, nsteps=steps, graph=False, timed=True) / steps
+        sim.step(dt=0.08, nsteps=20, timed=True)          # warm-up
+        ms_call = sim.step(dt=0.08, nsteps=steps, timed=True) / steps
+        ms_single = sum(sim.step(dt=0.08, nsteps=1, timed=True) for _ in range(steps)) / steps
         nr, nphi, nz = vol.shape
         orc = O.FluidSim(vol, disc.inner_radius, disc.outer_radius, falloff=disc.density_falloff)
         t0 = time.perf_counter()
         orc.step(dt=0.08, jacobi=8, nsteps=5, volume=True)
         cpu_ms = (time.perf_counter() - t0) * 1e3 / 5
-        # algorithmic bytes: every field read and written once per kernel, the texture written once
+        # algorithmic bytes of a single step: every field read and written once, the texture written once
         n = nr * nphi
         algo = (19 * n + n * nz) * 4
-        out[name] = {"us_per_step_graph": ms_graph * 1e3, "us_per_step_stream": ms_plain * 1e3,
-                     "launches_per_step": 4, "algorithmic_bytes_per_step": algo,
-                     "achieved_GBs_graph": algo / (ms_graph * 1e-3) / 1e9,
+        out[name] = {"us_per_step": ms_call * 1e3, "us_per_step_single_calls": ms_single * 1e3,
+                     "launches_per_call": 1, "algorithmic_bytes_per_step": algo,
+                     "achieved_GBs_single_calls": algo / (ms_single * 1e-3) / 1e9,
                      "oracle_cpu_ms_per_step_1_thread": cpu_ms,
-                     "speedup_vs_oracle": cpu_ms / ms_graph}
+                     "speedup_vs_oracle": cpu_ms / ms_call}
         sim.close()
         ctx.close()
     return out

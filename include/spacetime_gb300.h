@@ -338,7 +338,7 @@ void st_fluid_params_default(st_fluid_params* p);
 int st_fluid_create(st_fluid** out, st_context* ctx, const st_disc* disc, const st_fluid_params* p);
 /* nsteps steps of dt (step_sim! defaults: dt 0.05, jacobi 8, i.e.
  * 2 ceil(jacobi / 2) Jacobi sweeps), queued on the context's stream.
- * use_graph = 1 replays a CUDA graph of the step's launches; ms (may be
+ * The steps of a call are one launch whatever use_graph says; ms (may be
  * NULL) receives the device time of the steps (the call then waits for them). */
 int st_fluid_step(st_fluid* f, double dt, int jacobi, int nsteps, int use_graph, float* ms);
 /* Host copies of the solver state ((nr, nphi) column-major; any may be NULL):

@@ -7,36 +7,39 @@
 // One step of the reference is ~20 dispatches (src/disc_sim.jl:287-320):
 // velocity advection, forcing, divergence, 2 ceil(jacobi / 2) Jacobi sweeps,
 // gradient subtraction, forward and backward density advection, the
-// MacCormack combine and the extrusion.  Here it is four kernels:
+// MacCormack combine and the extrusion.  Here the steps of a call are one
+// cooperative launch (fluid_steps_kernel) of two phases a step:
 //
-//   fluid_velocity_kernel   advection of (vu, vv) under shear + itself, then
-//                           the curl-noise forcing, drag and edge taper of the
-//                           same cell (pointwise after the advection);
-//   fluid_divergence_kernel divergence of the forced field and the first
-//                           Jacobi sweep, which from p = 0 is -dv / 4;
-//   fluid_pressure_kernel   the remaining sweeps, temporally blocked: a tile
-//                           and a halo as wide as the sweeps it runs are
-//                           staged in shared memory and every sweep updates
-//                           the shrinking valid region there; the last pass
-//                           subtracts the pressure gradient on the tile;
-//   fluid_density_kernel    MacCormack advection of the surface density: the
-//                           forward result at the cell and at the four
-//                           corners of its backward point are recomputed in
-//                           registers (each is one bilinear sample), so the
-//                           forward and backward fields never go through
-//                           memory; then the limiter, the relaxation toward
-//                           the noise-modulated profile, and the extrusion of
-//                           the new value through the nz envelope cells.
+//   pressure   a tile and a halo as wide as its sweeps in shared memory: the
+//              divergence, every sweep on the shrinking valid region, and the
+//              gradient subtraction (in passes where the sweeps are many);
+//              blocks without a tile meanwhile evaluate the noise that the
+//              next phase needs, which depends on the clock alone;
+//   advection  MacCormack advection and relaxation of the surface density, and
+//              the next step's velocity advection and forcing, both of which
+//              need the projected velocity of all cells and nothing more.
+//              The forward density at the four corners of a cell's backward
+//              point is recomputed in registers, so the forward and backward
+//              fields never go through memory.
+//
+// The extrusion of the density through the nz envelope cells follows the last
+// step of a launch: the texture is read by later work of the stream only.
+//
+// What bounds it: a grid is some ten thousand cells, so a step is latency, not
+// work.  As four launches (velocity, divergence, pressure, density) a step
+// was 21 us, most of it launch and drain; the two grid barriers that are left
+// cost about 1.5 us each.  256 x 64 cells, 8 sweeps: 20.5 -> 8.9 us a step of
+// 100 in a call, 21.4 -> 16.3 us a single one.  Grids that fill the GPU several
+// times over take the same phases as launches of their own.
 //
 // Each cell's arithmetic is the reference's, in the same order, in float;
 // this unit is compiled without multiply-add contraction so every operation
 // rounds as written.  Index arithmetic is 1-based in the formulas, as in the
 // reference; field (i, j) lives at (i - 1) + nr (j - 1).
 //
-// The simulation clock lives on the device (t[parity] is read by the step,
-// t[1 - parity] = t[parity] + dt written by it) and the density ping-pongs
-// between two buffers by the same parity, so a step's launches are fixed per
-// (parity, dt, jacobi) and are captured once into a CUDA graph per parity.
+// The simulation clock lives on the device (a step of parity q reads t[q] and
+// leaves t[1 - q] = t[q] + dt) and the density ping-pongs between two buffers
+// by the same parity.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -119,7 +122,9 @@ __device__ __forceinline__ Foot footprint(float x, float y, int nr, int nphi) {
   return f;
 }
 
-__device__ __forceinline__ float bilerp(const float* __restrict__ f, const Foot& q) {
+// (plain pointers: the fields change within a launch, and the read-only path
+// could return what it held before a barrier)
+__device__ __forceinline__ float bilerp(const float* f, const Foot& q) {
   const float a = f[q.o00] + q.tx * (f[q.o10] - f[q.o00]);
   const float b = f[q.o01] + q.tx * (f[q.o11] - f[q.o01]);
   return a + q.ty * (b - a);
@@ -135,33 +140,77 @@ struct Fields {
   const float* base;            // radial profile (relaxation target)
   const float* shear;           // [nr] Keplerian shear, phi cells / M-time
   const float* env;             // [nr][nz] vertical envelope, (nr, nz) column-major
-  float* prs[2];                // pressure ping-pong
-  float* div;
+  float* prs[2];                // pressure ping-pong and
+  float* div;                   //   divergence, where the sweeps take several passes
+  float* fu; float* fv;         // the forcing's curl noise for the next velocity phase
+  float* tgt;                   // the relaxation target of the next density phase
   float* t;                     // [2] simulation clock by parity
+  unsigned* count;              // arrivals at the grid barrier, never reset
+  int* status;                  // set when a barrier's wait ran out
   float* vol;                   // (nr, nphi, nz) density texture of the context
 };
 
+constexpr int THREADS = 512, WARPS = THREADS / 32;
+constexpr int TI = 32;             // tile of the pressure phase along i (fastest)
+constexpr int LOW = 8, TALL = 32;  // and along j: in the one launch, in launches by phase
+// Sweeps per pass; halo = sweeps (+1 on the last pass).  The widest staged block
+// is then 64 cells along i: a thread owns one column of it, every eighth row.
+constexpr int MAX_SWEEPS = 15;
+constexpr int COLS = TI + 2 * (MAX_SWEEPS + 1), ROWS = THREADS / COLS;
+constexpr unsigned WAIT_LIMIT = 1u << 22;  // polls of a barrier, some seconds
+
+// Floats of shared memory of a pass: p twice.
+constexpr size_t tile_floats(int tj, int H) { return 2 * (size_t)(TI + 2 * H) * (tj + 2 * H); }
+static_assert(tile_floats(TALL, MAX_SWEEPS + 1) * sizeof(float) <= 48 * 1024, "no opt-in needed");
+
+// All blocks of the (cooperative) launch; `target` counts their arrivals since
+// the counter's creation, modulo 2^32.  False, for the whole block, when the
+// wait ran out; the fields are then not to be used.  (A word a block that every
+// block polls instead of one counter took 30,000 cycles: 152 x 152 polls.)
+__device__ __forceinline__ bool grid_barrier(const Fields& F, unsigned target) {
+  int out = 0;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    unsigned v;
+    asm volatile("atom.add.release.gpu.global.u32 %0, [%1], 1;" : "=r"(v) : "l"(F.count) : "memory");
+    unsigned polls = 0;
+    while (true) {
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(F.count) : "memory");
+      if ((int)(v - target) >= 0) break;
+      if (++polls >= WAIT_LIMIT) { out = 1; atomicExch(F.status, 1); break; }
+    }
+  }
+  return !__syncthreads_or(out);
+}
+
+// psi on a coarse lattice (~12-cell eddies) drifting in time; F = curl(psi z)
+// (k_force!, src/disc_sim.jl:150-172).
+constexpr float FORCE_SC = 0.085f, FORCE_E = 0.35f;
+__device__ __forceinline__ float force_u(int i, int j, float t) {
+  const float px = (float)i * FORCE_SC, py = (float)j * FORCE_SC, pz = t * 0.35f;
+  const float dpy = noise3(px, py + FORCE_E, pz) - noise3(px, py - FORCE_E, pz);
+  return dpy / (2.0f * FORCE_E);
+}
+__device__ __forceinline__ float force_v(int i, int j, float t) {
+  const float px = (float)i * FORCE_SC, py = (float)j * FORCE_SC, pz = t * 0.35f;
+  const float dpx = noise3(px + FORCE_E, py, pz) - noise3(px - FORCE_E, py, pz);
+  return -dpx / (2.0f * FORCE_E);
+}
+__device__ __forceinline__ float target(const Fields& F, int idx, int i, int j, float t) {
+  const float n = noise3((float)i * 0.11f, (float)j * 0.11f, t * 0.25f);
+  return F.base[idx] * expf(1.2f * (2.0f * n - 1.0f));
+}
+
 // Semi-Lagrangian velocity advection, then forcing + drag + edge taper
 // (k_advect_vel!, k_force!: src/disc_sim.jl:136-172).
-__global__ void fluid_velocity_kernel(Fields F, int parity, float dt, float amp, float drag) {
+__device__ __forceinline__ void velocity_cell(const Fields& F, int idx, int i, int j, float fu, float fv, float dt,
+                                              float amp, float drag) {
   const int nr = F.nr, nphi = F.nphi;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x + 1, j = blockIdx.y + 1;  // one grid row per phi row
-  if (i > nr) return;
-  const int idx = (i - 1) + nr * (j - 1);
   const float x = (float)i - dt * F.vu[idx];
   const float y = (float)j - dt * (F.vv[idx] + F.shear[i - 1]);
   const Foot q = footprint(x, y, nr, nphi);
   float u = bilerp(F.vu, q);
   float v = bilerp(F.vv, q);
-  // psi on a coarse lattice (~12-cell eddies) drifting in time; F = curl(psi z)
-  const float t = F.t[parity];
-  const float sc = 0.085f;
-  const float px = (float)i * sc, py = (float)j * sc, pz = t * 0.35f;
-  const float e = 0.35f;
-  const float dpy = noise3(px, py + e, pz) - noise3(px, py - e, pz);
-  const float dpx = noise3(px + e, py, pz) - noise3(px - e, py, pz);
-  const float fu = dpy / (2.0f * e);
-  const float fv = -dpx / (2.0f * e);
   float edge = fminf((float)i - 1.0f, (float)(nr - i)) * 0.125f;
   edge = fminf(fmaxf(edge, 0.0f), 1.0f);
   const float damp = expf(-drag * dt);
@@ -171,96 +220,89 @@ __global__ void fluid_velocity_kernel(Fields F, int parity, float dt, float amp,
   F.vv2[idx] = v;
 }
 
-// Divergence (k_div!) and the first Jacobi sweep from p = 0 (k_jacobi!:
-// 0.25 ((((0 + 0) + 0) + 0) - dv) = 0.25 (-dv)); with no sweeps p stays 0.
-__global__ void fluid_divergence_kernel(Fields F, int first_sweep) {
-  const int nr = F.nr, nphi = F.nphi;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x + 1, j = blockIdx.y + 1;
-  if (i > nr) return;
-  const int idx = (i - 1) + nr * (j - 1);
-  const int ip = min(i + 1, nr), im = max(i - 1, 1);
-  const int jp = jwrap(j, nphi) + 1, jm = jwrap(j - 2, nphi) + 1;
-  const float dv = 0.5f * (F.vu2[(ip - 1) + nr * (j - 1)] - F.vu2[(im - 1) + nr * (j - 1)] +
-                           F.vv2[(i - 1) + nr * (jp - 1)] - F.vv2[(i - 1) + nr * (jm - 1)]);
-  F.div[idx] = dv;
-  F.prs[0][idx] = first_sweep ? 0.25f * (0.0f - dv) : 0.0f;
-}
-
-constexpr int TI = 32, TJ = 8;     // tile of the blocked sweeps (i fastest)
-constexpr int MAX_SWEEPS = 16;     // sweeps per pass; halo = sweeps (+1 on the last pass): <= 33 KB of shared memory
-
-// `sweeps` Jacobi sweeps (k_jacobi!, src/disc_sim.jl:184-192) on one tile,
-// reading p from prs[src] and, unless `last`, writing the tile's p to
-// prs[1 - src]; the last pass subtracts the gradient (k_subgrad!,
-// src/disc_sim.jl:194-203) on the tile: (vu, vv) = (vu2, vv2) - grad p / 2.
-// Shared memory: p ping-pong and dv over the tile + halo.
-__global__ void __launch_bounds__(256) fluid_pressure_kernel(Fields F, int src, int sweeps, int last) {
-  extern __shared__ float sm[];
+// One tile's `sweeps` Jacobi sweeps (k_jacobi!, src/disc_sim.jl:184-192).  The
+// first pass forms the divergence (k_div!) and starts from the sweep from p = 0
+// (0.25 ((((0 + 0) + 0) + 0) - dv) = 0.25 (-dv)) or, with no sweeps at all, from
+// p = 0; later ones read p from prs[src].  The last pass subtracts the gradient
+// (k_subgrad!, src/disc_sim.jl:194-203): (vu, vv) = (vu2, vv2) - grad p / 2; the
+// others write p to prs[1 - src].  A thread keeps its cells' divergence in
+// registers over the sweeps, and no cell's place needs a division.
+template <int TJ>
+__device__ __forceinline__ void pressure_tile(const Fields& F, int bi, int bj, bool first, bool any, int src,
+                                              int sweeps, bool last, float* sm) {
   const int nr = F.nr, nphi = F.nphi;
   const int H = sweeps + (last ? 1 : 0);
-  const int RI = TI + 2 * H, RJ = TJ + 2 * H, RN = RI * RJ;
-  float* P0 = sm;
-  float* P1 = sm + RN;
-  float* D = sm + 2 * RN;
-  const int i0 = blockIdx.x * TI + 1 - H;  // global (unclamped) i of local row 0
-  const int j0 = blockIdx.y * TJ + 1 - H;
-  const float* __restrict__ pin = src ? F.prs[1] : F.prs[0];
-  float* __restrict__ pout = src ? F.prs[0] : F.prs[1];
-  // blockDim = (32, 8): x runs along i (coalesced), y along phi
-  const int tx = threadIdx.x, ty = threadIdx.y;
-  for (int lj = ty; lj < RJ; lj += 8) {
-    const int gj = jwrap(j0 + lj - 1, nphi) + 1;
-    for (int li = tx; li < RI; li += 32) {
-      const int gi = i0 + li;
-      float pv = 0.0f, dv = 0.0f;
-      if (gi >= 1 && gi <= nr) {
-        const int o = (gi - 1) + nr * (gj - 1);
-        pv = pin[o];
-        dv = F.div[o];
-      }
-      P0[li + RI * lj] = pv;
-      D[li + RI * lj] = dv;
+  const int RI = TI + 2 * H, RJ = TJ + 2 * H;
+  float* cur = sm;
+  float* nxt = sm + RI * RJ;
+  constexpr int MAX_CELLS = (TJ + 2 * (MAX_SWEEPS + 1) + ROWS - 1) / ROWS;
+  const int li = threadIdx.x % COLS, row = threadIdx.x / COLS;
+  const int gi = bi * TI + 1 - H + li;  // global i of the thread's column
+  const int j0 = bj * TJ - H;           // global (unwrapped, 0-based) j of local row 0
+  const bool in = li < RI && gi >= 1 && gi <= nr;
+  // clamped radial neighbours
+  const int up = gi + 1 <= nr ? 1 : 0, dn = gi - 1 >= 1 ? -1 : 0;
+  const int edge = in ? min(li, RI - 1 - li) : -1;
+  const bool mine = in && li >= H && li < H + TI;
+  const float* pin = src ? F.prs[1] : F.prs[0];
+  float* pout = src ? F.prs[0] : F.prs[1];
+  float D[MAX_CELLS], pv[MAX_CELLS];
+#pragma unroll
+  for (int c = 0; c < MAX_CELLS; ++c) {
+    const int lj = row + c * ROWS;
+    D[c] = pv[c] = 0.0f;
+    if (lj >= RJ || !in) continue;
+    const int j = jwrap(j0 + lj, nphi), o = (gi - 1) + nr * j;
+    if (first) {
+      const int jp = j + 1 < nphi ? o + nr : gi - 1, jm = j > 0 ? o - nr : (gi - 1) + nr * (nphi - 1);
+      D[c] = 0.5f * (F.vu2[o + up] - F.vu2[o + dn] + F.vv2[jp] - F.vv2[jm]);
+      if (any) pv[c] = 0.25f * (0.0f - D[c]);
+    } else {
+      D[c] = F.div[o];
+      pv[c] = pin[o];
     }
   }
+  float* at = cur + li + RI * row;  // the thread's cells lie ROWS rows apart
+#pragma unroll
+  for (int c = 0; c < MAX_CELLS; ++c)
+    if (li < RI && row + c * ROWS < RJ) at[c * ROWS * RI] = pv[c];
   __syncthreads();
-  float* cur = P0;
-  float* nxt = P1;
   for (int k = 1; k <= sweeps; ++k) {
     // valid region after this sweep: margin k from every side of the staged block
-    for (int lj = k + ty; lj < RJ - k; lj += 8) {
-      for (int li = k + tx; li < RI - k; li += 32) {
-        const int gi = i0 + li;
-        if (gi < 1 || gi > nr) continue;
-        const int lip = gi + 1 <= nr ? li + 1 : li;  // clamped radial neighbours
-        const int lim = gi - 1 >= 1 ? li - 1 : li;
-        const int l = li + RI * lj;
-        const float sum = cur[lip + RI * lj] + cur[lim + RI * lj] + cur[l + RI] + cur[l - RI];
-        nxt[l] = 0.25f * (sum - D[l]);
+    if (edge >= k) {
+      const float* a = cur + li + RI * row;
+      float* b = nxt + li + RI * row;
+#pragma unroll
+      for (int c = 0; c < MAX_CELLS; ++c) {
+        const int lj = row + c * ROWS;
+        if (lj < k || lj >= RJ - k) continue;
+        const float* p = a + c * ROWS * RI;
+        b[c * ROWS * RI] = 0.25f * (p[up] + p[dn] + p[RI] + p[-RI] - D[c]);
       }
     }
     __syncthreads();
     float* tmp = cur; cur = nxt; nxt = tmp;
   }
   // the tile's own cells
-  for (int tj = ty; tj < TJ; tj += 8) {
-    const int ti = tx;
-    const int gi = blockIdx.x * TI + 1 + ti, gjr = blockIdx.y * TJ + 1 + tj;
-    if (gi > nr || gjr > nphi) continue;
-    const int li = ti + H, lj = tj + H;
-    const int o = (gi - 1) + nr * (gjr - 1);
+#pragma unroll
+  for (int c = 0; c < MAX_CELLS; ++c) {
+    const int lj = row + c * ROWS;
+    if (!mine || lj < H || lj >= H + TJ || j0 + lj >= nphi) continue;
+    const int o = (gi - 1) + nr * (j0 + lj);
+    const float* p = cur + li + RI * lj;
     if (!last) {
-      pout[o] = cur[li + RI * lj];
+      pout[o] = p[0];
+      if (first) F.div[o] = D[c];
       continue;
     }
-    const int lip = gi + 1 <= nr ? li + 1 : li;
-    const int lim = gi - 1 >= 1 ? li - 1 : li;
-    F.vu[o] = F.vu2[o] - 0.5f * (cur[lip + RI * lj] - cur[lim + RI * lj]);
-    F.vv[o] = F.vv2[o] - 0.5f * (cur[li + RI * (lj + 1)] - cur[li + RI * (lj - 1)]);
+    F.vu[o] = F.vu2[o] - 0.5f * (p[up] - p[dn]);
+    F.vv[o] = F.vv2[o] - 0.5f * (p[RI] - p[-RI]);
   }
+  __syncthreads();
 }
 
 // Forward semi-Lagrangian density sample at cell (ci, cj) (k_adv_scalar!).
-__device__ __forceinline__ float advect_at(const Fields& F, const float* __restrict__ d, int ci, int cj, float dt) {
+__device__ __forceinline__ float advect_at(const Fields& F, const float* d, int ci, int cj, float dt) {
   const int o = (ci - 1) + F.nr * (cj - 1);
   const float x = (float)ci - dt * F.vu[o];
   const float y = (float)cj - dt * (F.vv[o] + F.shear[ci - 1]);
@@ -268,17 +310,12 @@ __device__ __forceinline__ float advect_at(const Fields& F, const float* __restr
 }
 
 // MacCormack density step + relaxation (k_adv_scalar! forward and backward,
-// k_maccormack!: src/disc_sim.jl:205-251) and the extrusion of the new value
-// through the envelope (k_extrude!, :253-266).  Thread 0 advances the clock.
-__global__ void fluid_density_kernel(Fields F, int parity, float dt, float relax) {
+// k_maccormack!: src/disc_sim.jl:205-251); returns the new value.
+__device__ __forceinline__ float density_cell(const Fields& F, int parity, int idx, int i, int j, float tgt, float dt,
+                                              float relax) {
   const int nr = F.nr, nphi = F.nphi;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x + 1, j = blockIdx.y + 1;
-  const float t = F.t[parity];
-  if (i == 1 && j == 1) F.t[1 - parity] = t + dt;
-  if (i > nr) return;
-  const int idx = (i - 1) + nr * (j - 1);
-  const float* __restrict__ d = parity ? F.dens[1] : F.dens[0];
-  float* __restrict__ dout = parity ? F.dens[0] : F.dens[1];
+  const float* d = parity ? F.dens[1] : F.dens[0];
+  float* dout = parity ? F.dens[0] : F.dens[1];
   // forward: d1 = d at the backtraced point; its corners bound the limiter
   const float x = (float)i - dt * F.vu[idx];
   const float y = (float)j - dt * (F.vv[idx] + F.shear[i - 1]);
@@ -297,24 +334,126 @@ __global__ void fluid_density_kernel(Fields F, int parity, float dt, float relax
   const float eb = c01 + qb.tx * (c11 - c01);
   const float d2 = ea + qb.ty * (eb - ea);
   const float a = fminf(fmaxf(d1 + 0.5f * (d[idx] - d2), lo), hi);
-  const float n = noise3((float)i * 0.11f, (float)j * 0.11f, t * 0.25f);
-  const float tgt = F.base[idx] * expf(1.2f * (2.0f * n - 1.0f));
   const float dn = fmaxf(a + relax * dt * (tgt - a), 0.0f);
   dout[idx] = dn;
-  // the envelope loads of a batch are issued before its stores, so the
-  // column's latency is paid once per eight cells rather than per cell
-  const size_t plane = (size_t)nr * nphi;
+  return dn;
+}
+
+// The envelope loads of a batch are issued before its stores, so the column's
+// latency is paid once per eight cells rather than per cell (k_extrude!,
+// src/disc_sim.jl:253-266).
+__device__ __forceinline__ void extrude(const Fields& F, int idx, int i, float dn) {
+  const size_t plane = (size_t)F.nr * F.nphi;
   const float* __restrict__ env = F.env + (i - 1);
   float* __restrict__ vol = F.vol + idx;
   int k = 0;
   for (; k + 8 <= F.nz; k += 8) {
     float e[8];
 #pragma unroll
-    for (int q = 0; q < 8; ++q) e[q] = __ldg(env + (size_t)nr * (k + q));
+    for (int q = 0; q < 8; ++q) e[q] = __ldg(env + (size_t)F.nr * (k + q));
 #pragma unroll
     for (int q = 0; q < 8; ++q) vol[plane * (k + q)] = dn * e[q];
   }
-  for (; k < F.nz; ++k) vol[plane * k] = dn * __ldg(env + (size_t)nr * k);
+  for (; k < F.nz; ++k) vol[plane * k] = dn * __ldg(env + (size_t)F.nr * k);
+}
+
+// `nsteps` steps from the state of `parity`; `sweeps` Jacobi sweeps each
+// (even, or 0); `base` barrier arrivals before this launch.  Work of a phase is
+// dealt in whole warps, round the blocks, so that a few hundred warps of work
+// occupy every SM.
+template <int BLOCKS_SM>
+__global__ void __launch_bounds__(THREADS, BLOCKS_SM)
+    fluid_steps_kernel(Fields F, int parity, int nsteps, float dt, int sweeps, float amp, float drag, float relax,
+                       unsigned base) {
+  extern __shared__ float sm[];
+  const unsigned nr = F.nr, n = nr * (unsigned)F.nphi;
+  const unsigned warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (*static_cast<volatile int*>(F.status)) return;  // an earlier launch's wait ran out
+  unsigned bars = base;
+  // f(kind, idx, i, j) for `kinds` kinds of work on every cell, by blocks b of nb
+  auto cells = [&](unsigned kinds, unsigned b, unsigned nb, auto f) {
+    const unsigned per = (n + 31) / 32, jobs = kinds * per;
+    for (unsigned w = warp * nb + b; w < jobs; w += WARPS * nb) {
+      const unsigned kind = w / per, idx = (w - kind * per) * 32 + lane;
+      if (idx >= n) continue;
+      const unsigned j = idx / nr;
+      f((int)kind, (int)idx, (int)(idx - j * nr) + 1, (int)j + 1);
+    }
+  };
+  const int gx = (F.nr + TI - 1) / TI, tiles = gx * ((F.nphi + LOW - 1) / LOW);
+  // blocks that have no tile evaluate the noise, if they are a fair share of the
+  // grid; else the advection does as it goes
+  const int spare = (int)gridDim.x - tiles;
+  const bool apart = spare * 4 >= (int)gridDim.x;
+  float t = parity ? F.t[1] : F.t[0];
+  cells(1, blockIdx.x, gridDim.x, [&](int, int idx, int i, int j) {
+    velocity_cell(F, idx, i, j, force_u(i, j, t), force_v(i, j, t), dt, amp, drag);
+  });
+  if (!grid_barrier(F, bars += gridDim.x)) return;
+  for (int k = 0; k < nsteps; ++k) {
+    const float tn = t + dt;
+    const bool end = k + 1 == nsteps;
+    if (blockIdx.x == 0 && threadIdx.x == 0) F.t[1 - parity] = tn;
+    int left = sweeps > 0 ? sweeps - 1 : 0, src = 0;
+    bool first = true;
+    while (true) {
+      const int m = min(left, MAX_SWEEPS);
+      left -= m;
+      for (int b = blockIdx.x; b < tiles; b += gridDim.x)
+        pressure_tile<LOW>(F, b % gx, b / gx, first, sweeps > 0, src, m, left == 0, sm);
+      if (left == 0) break;
+      if (!grid_barrier(F, bars += gridDim.x)) return;
+      src = 1 - src;
+      first = false;
+    }
+    if (apart && (int)blockIdx.x >= tiles)
+      cells(end ? 1 : 3, blockIdx.x - tiles, spare, [&](int kind, int idx, int i, int j) {
+        if (kind == 0) F.tgt[idx] = target(F, idx, i, j, t);
+        else if (kind == 1) F.fu[idx] = force_u(i, j, tn);
+        else F.fv[idx] = force_v(i, j, tn);
+      });
+    if (!grid_barrier(F, bars += gridDim.x)) return;
+    cells(end ? 1 : 2, blockIdx.x, gridDim.x, [&](int kind, int idx, int i, int j) {
+      if (kind == 0) {
+        const float dn =
+            density_cell(F, parity, idx, i, j, apart ? F.tgt[idx] : target(F, idx, i, j, t), dt, relax);
+        if (end) extrude(F, idx, i, dn);
+      } else {
+        velocity_cell(F, idx, i, j, apart ? F.fu[idx] : force_u(i, j, tn), apart ? F.fv[idx] : force_v(i, j, tn), dt,
+                      amp, drag);
+      }
+    });
+    if (!end && !grid_barrier(F, bars += gridDim.x)) return;
+    parity ^= 1;
+    t = tn;
+  }
+}
+
+// The phases as launches of their own, for grids that fill the GPU several times
+// over: a barrier's microsecond is nothing there, and blocks that come and go
+// keep the SMs fuller than a fixed few.  Blocks of the advection are 64 cells of
+// a phi row; its z is 0 for the density (`end`: and extrusion), 1 for the next
+// step's velocity.
+__global__ void __launch_bounds__(THREADS) fluid_pressure_kernel(Fields F, int parity, float dt, bool first, bool any,
+                                                                 int src, int sweeps, bool last) {
+  extern __shared__ float sm[];
+  if (first && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0)
+    F.t[1 - parity] = (parity ? F.t[1] : F.t[0]) + dt;
+  pressure_tile<TALL>(F, blockIdx.x, blockIdx.y, first, any, src, sweeps, last, sm);
+}
+__global__ void __launch_bounds__(64) fluid_advect_kernel(Fields F, int parity, int kind0, bool end, float dt,
+                                                          float amp, float drag, float relax) {
+  const int i = blockIdx.x * 64 + threadIdx.x + 1, j = blockIdx.y + 1;
+  if (i > F.nr) return;
+  const int idx = (i - 1) + F.nr * (j - 1);
+  if (blockIdx.z + kind0 == 0) {
+    const float dn = density_cell(F, parity, idx, i, j, target(F, idx, i, j, parity ? F.t[1] : F.t[0]), dt, relax);
+    if (end) extrude(F, idx, i, dn);
+  } else {
+    // the clock of the step to come: after a density phase's, or the call's first
+    const float t = (parity ^ (kind0 == 0 ? 1 : 0)) ? F.t[1] : F.t[0];
+    velocity_cell(F, idx, i, j, force_u(i, j, t), force_v(i, j, t), dt, amp, drag);
+  }
 }
 
 }  // namespace fluid
@@ -333,54 +472,73 @@ struct st_fluid {
   Fields F{};
   int parity = 0;
   double forcing = 6.0, drag = 0.15, relax = 0.05;
-  // graph per parity for the current (dt, jacobi)
-  cudaGraphExec_t exec[2] = {nullptr, nullptr};
-  const float* g_vol = nullptr;  // the density texture the graphs write
-  float g_dt = 0.f;
-  int g_jacobi = -1;
+  unsigned arrivals = 0;  // at the grid barrier, as the device counts them
+  int num_sms = 0;
   long long steps = 0;
 };
 
 namespace {
 
-int launch_step(st_fluid* f, int parity, float dt, int jacobi, cudaStream_t s) {
-  Fields F = f->F;
-  F.vol = nullptr;
-  st::CtxVolume cv;
-  if (st::context_volume(f->ctx, &cv) != ST_OK || !cv.on || cv.meta.nr != f->nr || cv.meta.nphi != f->nphi ||
-      cv.meta.nz != f->nz)
-    return ST_ESTATE;
-  F.vol = cv.d_vol;
-  // one 64-thread block per 64 cells of an s row, one grid row per phi row:
-  // the grids are a few tens of thousands of cells, so small blocks spread
-  // them over all SMs, and the 2-D grid gives (i, j) without a division
-  const int B = 64;
-  const dim3 G((f->nr + B - 1) / B, f->nphi);
-  fluid_velocity_kernel<<<G, B, 0, s>>>(F, parity, dt, (float)f->forcing, (float)f->drag);
-  // 2 ceil(jacobi / 2) sweeps (src/disc_sim.jl:305-308); the first runs in the
-  // divergence kernel, the rest in blocked passes of at most MAX_SWEEPS
-  const int total = jacobi > 0 ? 2 * ((jacobi + 1) / 2) : 0;
-  fluid_divergence_kernel<<<G, B, 0, s>>>(F, total > 0 ? 1 : 0);
-  int left = total > 0 ? total - 1 : 0;
-  int src = 0;
-  const dim3 grid((f->nr + TI - 1) / TI, (f->nphi + TJ - 1) / TJ);
-  do {
-    const int k = std::min(left, MAX_SWEEPS);
-    left -= k;
-    const int last = left == 0 ? 1 : 0;
-    const int H = k + last;
-    const size_t smem = 3 * (size_t)(TI + 2 * H) * (TJ + 2 * H) * sizeof(float);
-    fluid_pressure_kernel<<<grid, dim3(32, 8), smem, s>>>(F, src, k, last);
-    src = 1 - src;
-  } while (left > 0);
-  fluid_density_kernel<<<G, B, 0, s>>>(F, parity, dt, (float)f->relax);
-  return cudaGetLastError() == cudaSuccess ? ST_OK : ST_ECUDA;
-}
+constexpr int DENSE = 3;  // blocks an SM of the larger grids
+constexpr int LAUNCH_STEPS = 1024;  // steps of one launch, some milliseconds
 
-void drop_graphs(st_fluid* f) {
-  for (auto& e : f->exec)
-    if (e) { cudaGraphExecDestroy(e); e = nullptr; }
-  f->g_jacobi = -1;
+// `nsteps` (<= LAUNCH_STEPS) steps from the current parity on stream s.
+int launch_steps(st_fluid* f, float* vol, int nsteps, float dt, int jacobi, cudaStream_t s) {
+  Fields F = f->F;
+  F.vol = vol;
+  // 2 ceil(jacobi / 2) sweeps (src/disc_sim.jl:305-308)
+  int sweeps = jacobi > 0 ? 2 * ((jacobi + 1) / 2) : 0;
+  // the first sweep needs no neighbours; the rest run in passes of at most MAX_SWEEPS
+  const int rest = sweeps > 0 ? sweeps - 1 : 0;
+  const int passes = std::max(1, (rest + MAX_SWEEPS - 1) / MAX_SWEEPS);
+  // a block an SM, and no more than have two warps of cells, since the barriers'
+  // cost grows with the blocks; where there are more tiles, blocks for each and
+  // half as many for the noise; where the SMs do not hold those, launches by
+  // phase with taller tiles, which stage 2.3 cells for each of their own (8
+  // sweeps) and not 4.5.  us a step of 100: 192 x 256 cells 12.0 in one launch
+  // (22.0 as four launches a step), 1024 x 512 cells 62.8 in one, 46.6 by phase
+  // (61.5 as four)
+  const size_t cells = (size_t)f->nr * f->nphi;
+  const size_t gx = (f->nr + TI - 1) / TI, tiles = gx * ((f->nphi + LOW - 1) / LOW);
+  const size_t most = (size_t)f->num_sms * DENSE;
+  const int widest = std::min(rest, MAX_SWEEPS) + 1;
+  if (tiles > most) {
+    const dim3 ga((f->nr + 63) / 64, f->nphi, 1), gp(gx, (f->nphi + TALL - 1) / TALL);
+    const float amp = (float)f->forcing, drag = (float)f->drag, relax = (float)f->relax;
+    fluid_advect_kernel<<<ga, 64, 0, s>>>(F, f->parity, 1, false, dt, amp, drag, relax);
+    for (int k = 0; k < nsteps; ++k) {
+      const bool end = k + 1 == nsteps;
+      int left = rest;
+      for (int pass = 0; pass < passes; ++pass) {
+        const int m = std::min(left, MAX_SWEEPS);
+        left -= m;
+        fluid_pressure_kernel<<<gp, THREADS, tile_floats(TALL, widest) * sizeof(float), s>>>(
+            F, f->parity, dt, pass == 0, sweeps > 0, pass & 1, m, left == 0);
+      }
+      fluid_advect_kernel<<<dim3(ga.x, ga.y, end ? 1 : 2), 64, 0, s>>>(F, f->parity, 0, end, dt, amp, drag, relax);
+      f->parity ^= 1;
+    }
+    f->steps += nsteps;
+    return cudaGetLastError() == cudaSuccess ? ST_OK : ST_ECUDA;
+  }
+  const unsigned blocks = (unsigned)std::min(
+      most, std::max(std::min<size_t>(f->num_sms, (cells + 63) / 64), tiles + tiles / 2));
+  const void* kernel =
+      blocks > (unsigned)f->num_sms ? (const void*)fluid_steps_kernel<DENSE> : (const void*)fluid_steps_kernel<1>;
+  const size_t smem = tile_floats(LOW, widest) * sizeof(float);
+  int parity = f->parity;
+  float amp = (float)f->forcing, drag = (float)f->drag, relax = (float)f->relax;
+  unsigned base = f->arrivals;
+  void* args[] = {&F, &parity, &nsteps, &dt, &sweeps, &amp, &drag, &relax, &base};
+  if (cudaLaunchCooperativeKernel(kernel, dim3(blocks), dim3(THREADS), args, smem, s) !=
+      cudaSuccess) {
+    (void)cudaGetLastError();
+    return ST_ECUDA;
+  }
+  f->arrivals = base + blocks * (unsigned)nsteps * (unsigned)(passes + 1);
+  f->parity ^= nsteps & 1;
+  f->steps += nsteps;
+  return ST_OK;
 }
 
 }  // namespace
@@ -448,8 +606,11 @@ int st_fluid_create(st_fluid** out, st_context* ctx, const st_disc* disc, const 
   f->device = cv.device;
   f->nr = nr; f->nphi = nphi; f->nz = nz;
   f->forcing = fp->forcing; f->drag = fp->drag; f->relax = fp->relax;
-  // layout: vu vv vu2 vv2 dens0 dens1 base prs0 prs1 div (n each), env (nr nz), shear (nr), t (2)
-  const size_t total = 10 * n + (size_t)nr * nz + nr + 2;
+  // layout: vu vv vu2 vv2 dens0 dens1 base prs0 prs1 div fu fv tgt (n each), env (nr nz), shear (nr), t (2),
+  // count, status
+  bool up = cudaDeviceGetAttribute(&f->num_sms, cudaDevAttrMultiProcessorCount, f->device) == cudaSuccess;
+  if (!up) { delete f; return ST_ECUDA; }
+  const size_t total = 13 * n + (size_t)nr * nz + nr + 4;
   if (cudaStreamCreateWithFlags(&f->stream, cudaStreamNonBlocking) != cudaSuccess) { delete f; return ST_ECUDA; }
   if (cudaMalloc(&f->block, total * sizeof(float)) != cudaSuccess) {
     cudaStreamDestroy(f->stream);
@@ -463,9 +624,12 @@ int st_fluid_create(st_fluid** out, st_context* ctx, const st_disc* disc, const 
   F.dens[0] = b + 4 * n; F.dens[1] = b + 5 * n;
   float* base_d = b + 6 * n;
   F.prs[0] = b + 7 * n; F.prs[1] = b + 8 * n; F.div = b + 9 * n;
-  float* env_d = b + 10 * n;
+  F.fu = b + 10 * n; F.fv = b + 11 * n; F.tgt = b + 12 * n;
+  float* env_d = b + 13 * n;
   float* shear_d = env_d + (size_t)nr * nz;
   F.t = shear_d + nr;
+  F.count = reinterpret_cast<unsigned*>(F.t + 2);
+  F.status = reinterpret_cast<int*>(F.t + 3);
   F.base = base_d; F.env = env_d; F.shear = shear_d;
   bool ok = cudaMemsetAsync(b, 0, total * sizeof(float), f->stream) == cudaSuccess;
   ok = ok && cudaMemcpyAsync(F.dens[0], dens0.data(), n * sizeof(float), cudaMemcpyHostToDevice, f->stream) ==
@@ -487,7 +651,7 @@ int st_fluid_create(st_fluid** out, st_context* ctx, const st_disc* disc, const 
   return ST_OK;
 }
 
-int st_fluid_step(st_fluid* f, double dt, int jacobi, int nsteps, int use_graph, float* ms) {
+int st_fluid_step(st_fluid* f, double dt, int jacobi, int nsteps, int, float* ms) {
   if (!f || !(std::isfinite(dt)) || jacobi < 0 || jacobi > 4096 || nsteps < 0) return ST_EINVAL;
   if (ms) *ms = 0.f;
   if (cudaSetDevice(f->device) != cudaSuccess) return ST_ECUDA;
@@ -495,42 +659,20 @@ int st_fluid_step(st_fluid* f, double dt, int jacobi, int nsteps, int use_graph,
   if (st::context_volume(f->ctx, &cv) != ST_OK || !cv.on || cv.meta.nr != f->nr || cv.meta.nphi != f->nphi ||
       cv.meta.nz != f->nz)
     return ST_ESTATE;
-  const float dtf = (float)dt;
   // the steps run on the context's stream, so the next render sees the field
   cudaStream_t s = cv.stream;
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   if (ms && (cudaEventCreate(&e0) != cudaSuccess || cudaEventCreate(&e1) != cudaSuccess)) return ST_ECUDA;
   if (e0 && cudaEventRecord(e0, s) != cudaSuccess) return ST_ECUDA;
   int rc = ST_OK;
-  if (use_graph) {
-    if (f->g_jacobi != jacobi || f->g_dt != dtf || f->g_vol != cv.d_vol || f->exec[0] == nullptr) {
-      drop_graphs(f);
-      for (int par = 0; par < 2 && rc == ST_OK; ++par) {
-        cudaGraph_t g = nullptr;
-        if (cudaStreamBeginCapture(f->stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess) { rc = ST_ECUDA; break; }
-        const int lr = launch_step(f, par, dtf, jacobi, f->stream);
-        const cudaError_t ce = cudaStreamEndCapture(f->stream, &g);
-        if (lr != ST_OK || ce != cudaSuccess) { rc = lr != ST_OK ? lr : ST_ECUDA; if (g) cudaGraphDestroy(g); break; }
-        if (cudaGraphInstantiate(&f->exec[par], g, 0) != cudaSuccess) rc = ST_ECUDA;
-        cudaGraphDestroy(g);
-      }
-      if (rc != ST_OK) drop_graphs(f);
-      else { f->g_dt = dtf; f->g_jacobi = jacobi; f->g_vol = cv.d_vol; }
-    }
-    for (int k = 0; k < nsteps && rc == ST_OK; ++k) {
-      if (cudaGraphLaunch(f->exec[f->parity], s) != cudaSuccess) rc = ST_ECUDA;
-      else f->parity ^= 1;
-    }
-  } else {
-    for (int k = 0; k < nsteps && rc == ST_OK; ++k) {
-      rc = launch_step(f, f->parity, dtf, jacobi, s);
-      if (rc == ST_OK) f->parity ^= 1;
-    }
-  }
-  if (rc == ST_OK) f->steps += nsteps;
+  for (int left = nsteps; left > 0 && rc == ST_OK; left -= LAUNCH_STEPS)
+    rc = launch_steps(f, cv.d_vol, std::min(left, LAUNCH_STEPS), (float)dt, jacobi, s);
   if (e1) {
+    int status = 0;
     if (cudaEventRecord(e1, s) != cudaSuccess || cudaEventSynchronize(e1) != cudaSuccess) rc = ST_ECUDA;
     else if (cudaEventElapsedTime(ms, e0, e1) != cudaSuccess) { (void)cudaGetLastError(); *ms = 0.f; }
+    if (cudaMemcpy(&status, f->F.status, sizeof status, cudaMemcpyDeviceToHost) != cudaSuccess || status != 0)
+      rc = ST_ECUDA;
   }
   if (e0) cudaEventDestroy(e0);
   if (e1) cudaEventDestroy(e1);
@@ -544,7 +686,7 @@ int st_fluid_state(st_fluid* f, float* vu, float* vv, float* dens, float* volume
   if (st::context_volume(f->ctx, &cv) != ST_OK) return ST_ESTATE;
   cudaStream_t s = cv.stream;
   const size_t n = (size_t)f->nr * f->nphi;
-  float tt[2] = {0.f, 0.f};
+  struct { float t[2]; unsigned count; int status; } tail{};  // as they lie
   bool ok = true;
   if (vu) ok = ok && cudaMemcpyAsync(vu, f->F.vu, n * sizeof(float), cudaMemcpyDeviceToHost, s) == cudaSuccess;
   if (vv) ok = ok && cudaMemcpyAsync(vv, f->F.vv, n * sizeof(float), cudaMemcpyDeviceToHost, s) == cudaSuccess;
@@ -556,17 +698,16 @@ int st_fluid_state(st_fluid* f, float* vu, float* vv, float* dens, float* volume
     ok = ok && cudaMemcpyAsync(volume, cv.d_vol, n * f->nz * sizeof(float), cudaMemcpyDeviceToHost, s) ==
                    cudaSuccess;
   }
-  ok = ok && cudaMemcpyAsync(tt, f->F.t, sizeof tt, cudaMemcpyDeviceToHost, s) == cudaSuccess;
+  ok = ok && cudaMemcpyAsync(&tail, f->F.t, sizeof tail, cudaMemcpyDeviceToHost, s) == cudaSuccess;
   ok = ok && cudaStreamSynchronize(s) == cudaSuccess;
-  if (!ok) return ST_ECUDA;
-  if (t) *t = (double)tt[f->parity];
+  if (!ok || tail.status != 0) return ST_ECUDA;
+  if (t) *t = (double)tail.t[f->parity];
   return ST_OK;
 }
 
 void st_fluid_destroy(st_fluid* f) {
   if (!f) return;
   cudaSetDevice(f->device);
-  drop_graphs(f);
   if (f->stream) cudaStreamSynchronize(f->stream);
   cudaFree(f->block);
   if (f->stream) cudaStreamDestroy(f->stream);
