@@ -972,73 +972,91 @@ __device__ __forceinline__ R disc_exact(const TraceParams& p, R xh, R yh, R pxh,
   return T_obs / T_emit;
 }
 
+// One gas sample's absorption, radiance and colour (src/metal.jl:1455-1500), at
+// fraction fs of the step yp -> yn; false where there is nothing to blend.
+template <typename R>
+struct GasSample {
+  R aa, inte;
+  float4 col;
+};
+template <typename R>
+__device__ __forceinline__ bool gas_sample(const TraceParams& p, const R* yp, const R* yn, R fs, R sx, R sy, R sz,
+                                           R scyl, R pt, R scam, GasSample<R>* o) {
+  const R r_isco = PR(r_isco), M = PR(M);
+  const R phi = atan2_(sy, sx);
+  R rho = sample_volume(p, scyl, phi, sz);
+  if (!(rho > R(1e-4))) return false;
+  R T_emit;
+  if constexpr (IsD<R>::v) {
+    const R Rr = max_(scyl, r_isco) / (R(2) * M);
+    T_emit = exp_(R(10.034259) - R(0.375) * log_(max_(Rr * Rr, R(1e-6))));
+  } else {
+    // base 2: exp(c - 0.375 ln Rr^2) = 2^(c log2(e) - 0.75 log2 Rr)
+    const float Rr = fmaxf(scyl, r_isco) * p.f.inv_2m;
+    T_emit = ex2_(fmaf(-0.75f, lg2_(fmaxf(Rr, 1e-3f)), float(10.034259 * kLog2e)));
+  }
+  if (scyl < r_isco) { const R t3 = scyl / r_isco; rho *= t3 * t3 * t3; }
+  const R psx = yp[3] + fs * (yn[3] - yp[3]);
+  const R psy = yp[4] + fs * (yn[4] - yp[4]);
+  const R opz = emitter_opz(sx, sy, psx, psy, -pt, M, PR(a), r_isco, PR(E_isco), PR(L_isco));
+  const R T_obs = T_emit * scam / opz;
+  o->col = lut_color(p, T_obs, false);
+  if constexpr (IsD<R>::v) {
+    o->inte = R(100) / (exp_(R(29622.4) / max_(T_obs, R(1))) - R(1));
+    const R tau = PR(opac) * rho * PR(ds_gas);
+    o->aa = R(1) - exp_(-tau);
+  } else {
+    // 100 emis / (exp(29622.4 / T) - 1) and 1 - exp(-opac rho ds) in base 2,
+    // the products of constants from the host
+    o->inte = p.f.emis100 * rcp_(ex2_(float(29622.4 * kLog2e) * rcp_(fmaxf(T_obs, 1.f))) - 1.f);
+    o->aa = 1.f - ex2_(-(rho * p.f.opds_l2));
+  }
+  return true;
+}
+template <typename R>
+__device__ __forceinline__ void blend_sample(const TraceParams& p, const GasSample<R>& o, R* acc, R* alpha) {
+  R w = *alpha * o.aa * o.inte;
+  if constexpr (IsD<R>::v) w = w * PR(emis);
+  acc[0] += w * R(o.col.x); acc[1] += w * R(o.col.y); acc[2] += w * R(o.col.z);
+  *alpha *= (R(1) - o.aa);
+}
+
 // Gas march along one accepted step, src/metal.jl:1429-1513.  Returns true
 // when the transmittance is exhausted.
-template <typename R>
-__device__ __forceinline__ bool march_gas(const TraceParams& p, const R* yp, const R* yn, R r2p, R h_used, R vlen,
-                                          RayState<R>& st) {
-  const R r2n = yn[0] * yn[0] + yn[1] * yn[1] + yn[2] * yn[2];
-  if (!(st.alpha > R(0.003) && min_(r2p, r2n) < PR(vol_rb2))) return false;
-  const R ds = PR(ds_gas);
-  const R seg = h_used * vlen;
-  // a step spans at most a few M of arc; anything else (overflow, NaN) is not marched
-  if (!(seg < R(64))) return false;
-  R t_s = ds - st.march_acc;
-  if (t_s > seg) { st.march_acc += seg; return false; }
-  const R zmax = PR(zmax);
-  const R r_isco = PR(r_isco), M = PR(M);
-  const R inv_seg = R(1) / seg;
-  // bounded: seg < 64 and ds >= dt, so at most 64/dt + 1 samples (capped at 8192)
-  for (int guard = 0; guard < 8192 && t_s <= seg && st.alpha > R(0.003); ++guard) {
-    const R fs = IsD<R>::v ? t_s / seg : t_s * inv_seg;
-    const R sx = yp[0] + fs * (yn[0] - yp[0]);
-    const R sy = yp[1] + fs * (yn[1] - yp[1]);
-    const R sz = yp[2] + fs * (yn[2] - yp[2]);
-    if (fabs_(sz) < zmax) {
-      const R scyl = sqrt_(sx * sx + sy * sy);
-      if (scyl > R(1e-6)) {
-        const R phi = atan2_(sy, sx);
-        R rho = sample_volume(p, scyl, phi, sz);
-        ++st.gas;
-        if (rho > R(1e-4)) {
-          R T_emit;
-          if constexpr (IsD<R>::v) {
-            const R Rr = max_(scyl, r_isco) / (R(2) * M);
-            T_emit = exp_(R(10.034259) - R(0.375) * log_(max_(Rr * Rr, R(1e-6))));
-          } else {
-            // base 2: exp(c - 0.375 ln Rr^2) = 2^(c log2(e) - 0.75 log2 Rr)
-            const float Rr = fmaxf(scyl, r_isco) * p.f.inv_2m;
-            T_emit = ex2_(fmaf(-0.75f, lg2_(fmaxf(Rr, 1e-3f)), float(10.034259 * kLog2e)));
-          }
-          if (scyl < r_isco) { const R t3 = scyl / r_isco; rho *= t3 * t3 * t3; }
-          const R psx = yp[3] + fs * (yn[3] - yp[3]);
-          const R psy = yp[4] + fs * (yn[4] - yp[4]);
-          const R opz = emitter_opz(sx, sy, psx, psy, -st.pt, M, PR(a), r_isco, PR(E_isco), PR(L_isco));
-          const R T_obs = T_emit * st.scam / opz;
-          const float4 col = lut_color(p, T_obs, false);
-          R aa, w;
-          if constexpr (IsD<R>::v) {
-            const R inten = R(100) / (exp_(R(29622.4) / max_(T_obs, R(1))) - R(1));
-            const R tau = PR(opac) * rho * ds;
-            aa = R(1) - exp_(-tau);
-            w = st.alpha * aa * inten * PR(emis);
-          } else {
-            // 100 emis / (exp(29622.4 / T) - 1) and 1 - exp(-opac rho ds) in base 2,
-            // the products of constants from the host
-            const float inte = p.f.emis100 * rcp_(ex2_(float(29622.4 * kLog2e) * rcp_(fmaxf(T_obs, 1.f))) - 1.f);
-            aa = 1.f - ex2_(-(rho * p.f.opds_l2));
-            w = st.alpha * aa * inte;
-          }
-          st.acc[0] += w * R(col.x); st.acc[1] += w * R(col.y); st.acc[2] += w * R(col.z);
-          st.alpha *= (R(1) - aa);
+struct MarchGas {
+  template <typename R>
+  __device__ __forceinline__ bool operator()(const TraceParams& p, const R* yp, const R* yn, R r2p, R h_used, R vlen,
+                                             RayState<R>& st) const {
+    const R r2n = yn[0] * yn[0] + yn[1] * yn[1] + yn[2] * yn[2];
+    if (!(st.alpha > R(0.003) && min_(r2p, r2n) < PR(vol_rb2))) return false;
+    const R ds = PR(ds_gas);
+    const R seg = h_used * vlen;
+    // a step spans at most a few M of arc; anything else (overflow, NaN) is not marched
+    if (!(seg < R(64))) return false;
+    R t_s = ds - st.march_acc;
+    if (t_s > seg) { st.march_acc += seg; return false; }
+    const R inv_seg = R(1) / seg;
+    // bounded: seg < 64 and ds >= dt, so at most 64/dt + 1 samples (capped at 8192)
+    for (int guard = 0; guard < 8192 && t_s <= seg && st.alpha > R(0.003); ++guard) {
+      const R fs = IsD<R>::v ? t_s / seg : t_s * inv_seg;
+      const R sx = yp[0] + fs * (yn[0] - yp[0]);
+      const R sy = yp[1] + fs * (yn[1] - yp[1]);
+      const R sz = yp[2] + fs * (yn[2] - yp[2]);
+      if (fabs_(sz) < PR(zmax)) {
+        const R scyl = sqrt_(sx * sx + sy * sy);
+        if (scyl > R(1e-6)) {
+          ++st.gas;
+          GasSample<R> o;
+          if (gas_sample(p, yp, yn, fs, sx, sy, sz, scyl, st.pt, st.scam, &o))
+            blend_sample(p, o, st.acc, &st.alpha);
         }
       }
+      t_s += ds;
     }
-    t_s += ds;
+    st.march_acc = seg - (t_s - ds);
+    return st.alpha < R(0.003);
   }
-  st.march_acc = seg - (t_s - ds);
-  return st.alpha < R(0.003);
-}
+};
 
 // Tsitouras (2011) 5(4) pair, FSAL (published tableau).
 struct Tsit5C {
@@ -1186,12 +1204,22 @@ __device__ __forceinline__ void null_renorm(float* y, float* lo, float ptf, cons
 // ST_RAY_DEFER with its state as it entered the call (the only field the
 // call has written, r_prev, is rewritten to the same value when the step is
 // taken again), so the resume kernel can take it in a dense FP64 warp.
-template <int PREC, int KERR, int VOL, int SEM, int ORD = 4, int DEPTH = 0, int DEFER = 0>
-__device__ __forceinline__ bool step_ray(const TraceParams& p, RayState<typename RealOf<PREC>::T>& st) {
+// The gas along a step is `gas`'s to march (VOL; true ends the ray).
+template <int PREC, int KERR, int VOL, int SEM, int ORD = 4, int DEPTH = 0, int DEFER = 0, class Gas = MarchGas>
+__device__ __forceinline__ bool step_ray(const TraceParams& p, RayState<typename RealOf<PREC>::T>& st,
+                                         const Gas& gas = Gas{}) {
   using R = typename RealOf<PREC>::T;
   const R M = PR(M), a = PR(a);
   R* y = st.y;
-  const R r2 = y[0] * y[0] + y[1] * y[1] + y[2] * y[2];
+  // LATE, where the chain from step to step is the kernel's time (a gas that is
+  // marched elsewhere): the tests before a step only note why the ray ends, and
+  // one branch behind the step acts on it; the ray takes its last step in vain.
+  // 64x36 Kerr gas 1.09 -> 1.01 ms; frames that fill the GPU gain nothing by it.
+  constexpr bool LATE = !std::is_same<Gas, MarchGas>::value;
+  static_assert(!LATE || (PREC == ST_PREC_FP32 && ORD == 4 && SEM == ST_SEM_DRAFT && !DEPTH), "plain float steps");
+  // (LATE: the contraction that the compiler gives the other form, so that a ray
+  // takes the same steps; written out there too it cost the disc kernel 2.6 %)
+  const R r2 = LATE ? fma(y[2], y[2], fma(y[0], y[0], y[1] * y[1])) : y[0] * y[0] + y[1] * y[1] + y[2] * y[2];
   const R r = sqrt_(r2);
   R rk2 = r2;
   if constexpr (!KERR && SEM == ST_SEM_DRAFT) {
@@ -1207,8 +1235,21 @@ __device__ __forceinline__ bool step_ray(const TraceParams& p, RayState<typename
       st.r_layer_prev = r;
     }
   }
-  if (st.steps >= st.nmax) { st.flags |= ST_RAY_BUDGET; return true; }
-  if constexpr (SEM == ST_SEM_DRAFT) {
+  int end = 0;
+  if constexpr (LATE) {
+    if constexpr (KERR) {
+      rk2 = ks_r2(y[0], y[1], y[2], a);
+      end = rk2 < PR(rkill2) ? ST_RAY_CAPTURED : r > st.r_esc ? ST_RAY_ESCAPED : 0;
+    } else {
+      const bool near = r < R(3.2) * M;
+      const bool in = near && (r < st.r_floor || (r < R(2.95) * M && st.r_prev > R(0) && r < st.r_prev - R(1e-4) * M));
+      end = in ? ST_RAY_CAPTURED : r > st.r_esc ? ST_RAY_ESCAPED : 0;
+      if (near) st.r_prev = r;
+    }
+    if (st.steps >= st.nmax) end = ST_RAY_BUDGET;
+  } else if (st.steps >= st.nmax) { st.flags |= ST_RAY_BUDGET; return true; }
+  if constexpr (LATE) {
+  } else if constexpr (SEM == ST_SEM_DRAFT) {
     if constexpr (KERR) {
       rk2 = ks_r2(y[0], y[1], y[2], a);
       if (rk2 < PR(rkill2)) { st.flags |= ST_RAY_CAPTURED; return true; }
@@ -1317,6 +1358,14 @@ __device__ __forceinline__ bool step_ray(const TraceParams& p, RayState<typename
         const float2 o = add2(pk(y[2 * k], y[2 * k + 1]), pk(inc[2 * k], inc[2 * k + 1]));
         y[2 * k] = o.x; y[2 * k + 1] = o.y;
       }
+      if constexpr (LATE) {
+        if (end) {
+#pragma unroll
+          for (int k = 0; k < 6; ++k) y[k] = yp[k];
+          st.flags |= end;
+          return true;
+        }
+      }
     } else {
 #pragma unroll
       for (int k = 0; k < 6; ++k) y[k] = y[k] + inc[k];
@@ -1332,7 +1381,7 @@ __device__ __forceinline__ bool step_ray(const TraceParams& p, RayState<typename
     const R vlen = max_(sqrt_(k1[0] * k1[0] + k1[1] * k1[1] + k1[2] * k1[2]), R(1e-20));
     if constexpr (DEPTH) st.ell += h * vlen;
     if constexpr (VOL) {
-      const bool opaque = march_gas(p, yp, y, r2, h, vlen, st);
+      const bool opaque = gas(p, yp, y, r2, h, vlen, st);
       if constexpr (DEPTH) flush_bucket(p, st.pix, st.ell, st.acc);
       if (opaque) return true;
     } else {
