@@ -330,8 +330,8 @@ struct st_context {
   bool fan_valid = false;
   cudaStream_t side = nullptr;  // the fine fan runs here, beside the layer pass
   cudaEvent_t ev_coarse = nullptr, ev_fine = nullptr;
-  cudaStream_t ring = nullptr;  // the ring pass runs here, beside the layer pass
-  cudaEvent_t ev_pass = nullptr, ev_ring = nullptr;
+  cudaStream_t lstream = nullptr;  // the layer pass runs here, beside the ring pass
+  cudaEvent_t ev_pass = nullptr, ev_layer = nullptr;
   // adaptive refinement: per-pixel luminance moments, the flagged box
   float4* d_stat = nullptr;
   size_t stat_cap = 0;
@@ -1164,9 +1164,9 @@ int layered_render(st_context* ctx, const st_camera* cam, const st_spacetime* st
   const int rw = ring.width > 0 ? ring.width : rp->width, rh = ring.height > 0 ? ring.height : rp->height;
   if (use_ring && (rw < 2 || rh < 2 || (long long)rw * rh > (1ll << 30))) return ST_EINVAL;
   if (use_ring && (rc = ensure(&ctx->d_ring, &ctx->ring_cap, (size_t)rw * rh)) != ST_OK) return rc;
-  if (use_ring && !ctx->ring && cudaStreamCreateWithFlags(&ctx->ring, cudaStreamNonBlocking) != cudaSuccess)
+  if (use_ring && !ctx->lstream && cudaStreamCreateWithFlags(&ctx->lstream, cudaStreamNonBlocking) != cudaSuccess)
     return ST_ECUDA;
-  for (cudaEvent_t* e : {&ctx->ev_pass, &ctx->ev_ring})
+  for (cudaEvent_t* e : {&ctx->ev_pass, &ctx->ev_layer})
     if (use_ring && !*e && cudaEventCreateWithFlags(e, cudaEventDisableTiming) != cudaSuccess) return ST_ECUDA;
   ST_CUDA(cudaMemsetAsync(ctx->d_counters, 0, st::CNT_N * sizeof(unsigned long long), s));
   ST_CUDA(cudaEventRecord(ctx->ev0, s));
@@ -1203,33 +1203,42 @@ int layered_render(st_context* ctx, const st_camera* cam, const st_spacetime* st
       st::fill_float_copies(&lp);
       st::Variant lv = v;
       lv.sched = ST_SCHED_PIXEL;
-      // the fan is made and the pass before has read both layers
-      if (use_ring) ST_CUDA(cudaEventRecord(ctx->ev_pass, s));
-      ST_CUDA(st::launch_trace(lv, lp, rp->block_x, rp->block_y, ctx->num_sms, s));
-      ++launches;
-      cp.layer = ctx->d_layer;
+      int bx = rp->block_x, by = rp->block_y;  // launch_variant's rule for the tile shape
+      if (bx <= 0 || by <= 0 || bx * by != 128) { bx = 16; by = 8; }
+      if ((rc = ensure_tile_order(ctx, cam, lw, lh, bx, by, s, &lp.tile_order)) != ST_OK) return rc;
+      cudaStream_t ls = s;
       if (use_ring) {
-        // a finer layer of the wound rays only, over the box that can hold them;
-        // on a stream beside the layer pass, since each ends on a few rays that
-        // wind for a millisecond while most of the chip is idle
-        ST_CUDA(cudaStreamWaitEvent(ctx->ring, ctx->ev_pass, 0));
-        ST_CUDA(st::launch_fill_transparent(ctx->d_ring, (size_t)rw * rh, ctx->ring));
+        // a finer layer of the wound rays only, over the box that can hold them.
+        // It and the layer pass each end on a few rays that wind for a millisecond
+        // while most of the chip is idle, so they run side by side: the ring, whose
+        // rays are the longest, on the stream that the fan is made on, and the
+        // layer, centre first, on one that waits for the fan and so comes second.
+        ls = ctx->lstream;
+        ST_CUDA(st::launch_fill_transparent(ctx->d_ring, (size_t)rw * rh, s));
+        ST_CUDA(cudaEventRecord(ctx->ev_pass, s));
         TraceParams rq = lp;
         rq.width = rw;
         rq.height = rh;
         rq.ring_rmin = ring.rmin;
         rq.out = ctx->d_ring;
+        rq.tile_order = nullptr;
         rq.box_col0 = box.c0; rq.box_cols = box.cols;
         rq.box_row0 = box.r0; rq.box_rows = box.rows;
-        ST_CUDA(st::launch_trace(lv, rq, rp->block_x, rp->block_y, ctx->num_sms, ctx->ring));
-        ST_CUDA(cudaEventRecord(ctx->ev_ring, ctx->ring));
-        ST_CUDA(cudaStreamWaitEvent(s, ctx->ev_ring, 0));
+        ST_CUDA(st::launch_trace(lv, rq, rp->block_x, rp->block_y, ctx->num_sms, s));
+        ST_CUDA(cudaStreamWaitEvent(ls, ctx->ev_pass, 0));
         launches += 2;
         cp.ring = ctx->d_ring;
         cp.rw = rw;
         cp.rh = rh;
         cp.ring_rmin = (float)ring.rmin;
       }
+      ST_CUDA(st::launch_trace(lv, lp, rp->block_x, rp->block_y, ctx->num_sms, ls));
+      if (use_ring) {
+        ST_CUDA(cudaEventRecord(ctx->ev_layer, ls));
+        ST_CUDA(cudaStreamWaitEvent(s, ctx->ev_layer, 0));
+      }
+      ++launches;
+      cp.layer = ctx->d_layer;
     }
     p.out = ctx->d_fb;
     p.diag = host_diag ? ctx->d_diag : nullptr;
@@ -1476,8 +1485,8 @@ void st_context_destroy(st_context* ctx) {
   if (ctx->ev_fine) cudaEventDestroy(ctx->ev_fine);
   if (ctx->side) cudaStreamDestroy(ctx->side);
   if (ctx->ev_pass) cudaEventDestroy(ctx->ev_pass);
-  if (ctx->ev_ring) cudaEventDestroy(ctx->ev_ring);
-  if (ctx->ring) cudaStreamDestroy(ctx->ring);
+  if (ctx->ev_layer) cudaEventDestroy(ctx->ev_layer);
+  if (ctx->lstream) cudaStreamDestroy(ctx->lstream);
   cudaFree(ctx->d_vol);
   cudaFree(ctx->d_fb);
   cudaFree(ctx->d_rgb);
