@@ -275,6 +275,10 @@ static void shuffle(std::vector<int>& v, Rng& r) {
 // Context.
 // ---------------------------------------------------------------------------
 
+// Passes of a frame that run beside its first.
+constexpr int PASS_LANES = 3;
+constexpr size_t PASS_PIXELS = (size_t)1 << 23;  // of a frame whose passes do (0.4 GB of buffers)
+
 struct st_context {
   int device = 0;
   int num_sms = 0;
@@ -332,6 +336,12 @@ struct st_context {
   cudaEvent_t ev_coarse = nullptr, ev_fine = nullptr;
   cudaStream_t lstream = nullptr;  // the layer pass runs here, beside the ring pass
   cudaEvent_t ev_pass = nullptr, ev_layer = nullptr;
+  // the passes of a frame beside its first: a stream and a frame buffer each,
+  // the pass's end and its addition to the frame
+  cudaStream_t pstream[PASS_LANES] = {};
+  float4* d_pass[PASS_LANES] = {};
+  size_t pass_cap[PASS_LANES] = {};
+  cudaEvent_t ev_open = nullptr, ev_passed[PASS_LANES] = {}, ev_added[PASS_LANES] = {};
   // adaptive refinement: per-pixel luminance moments, the flagged box
   float4* d_stat = nullptr;
   size_t stat_cap = 0;
@@ -673,6 +683,31 @@ __global__ void scale_box_kernel(float4* fb, int W, int c0, int r0, int cols, in
   o.x *= s; o.y *= s; o.z *= s;
 }
 
+// A pass of its own buffer onto the frame: what the trace kernels do to the
+// frame before them, emission added and transmittance replaced.
+__global__ void add_pass_kernel(float4* __restrict__ fb, const float4* __restrict__ pass, size_t n) {
+  const size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= n) return;
+  float4 o = pass[k];
+  const float4 prev = fb[k];
+  o.x += prev.x; o.y += prev.y; o.z += prev.z;
+  fb[k] = o;
+}
+
+// Streams, events and buffers for the passes beside a frame's first.
+int ensure_pass_lanes(st_context* ctx, size_t npix, int lanes) {
+  if (!ctx->ev_open && cudaEventCreateWithFlags(&ctx->ev_open, cudaEventDisableTiming) != cudaSuccess) return ST_ECUDA;
+  for (int l = 0; l < lanes; ++l) {
+    if (!ctx->pstream[l] && cudaStreamCreateWithFlags(&ctx->pstream[l], cudaStreamNonBlocking) != cudaSuccess)
+      return ST_ECUDA;
+    for (cudaEvent_t* e : {&ctx->ev_passed[l], &ctx->ev_added[l]})
+      if (!*e && cudaEventCreateWithFlags(e, cudaEventDisableTiming) != cudaSuccess) return ST_ECUDA;
+    const int rc = ensure(&ctx->d_pass[l], &ctx->pass_cap[l], npix);
+    if (rc != ST_OK) return rc;
+  }
+  return ST_OK;
+}
+
 // Iteration budget of the persistent kernel's outer loop: enough for every
 // ray of the launch to take its whole step budget in chunk-sized slices.  The
 // environment variable SPACETIME_GB300_QUEUE_BUDGET=<n> lowers it to n, so a
@@ -797,6 +832,10 @@ int do_render(st_context* ctx, const st_camera* cam, const st_spacetime* stp, co
     p.stat = ctx->d_stat;
   }
   int launches = 0;
+  cudaStream_t ps = s;  // the stream of the pass being launched
+  // the launch's grid (launch_variant's rule for the tile shape)
+  int tile_x = rp->block_x, tile_y = rp->block_y;
+  if (tile_x <= 0 || tile_y <= 0 || tile_x * tile_y != 128) { tile_x = 16; tile_y = 8; }
   auto run_pass = [&](const PassPlan& pp, bool first) -> int {
     p.ju = pp.ju; p.jv = pp.jv; p.jw = pp.jw; p.jseed = pp.jseed;
     p.lens_u0 = pp.lens_u0; p.lens_v0 = pp.lens_v0; p.lens_w = pp.lens_w; p.lens_seed = pp.lens_seed;
@@ -838,17 +877,57 @@ int do_render(st_context* ctx, const st_camera* cam, const st_spacetime* stp, co
     }
     p.tile_order = nullptr;
     if (v.sched == ST_SCHED_PIXEL && !p.pix_list && p.box_cols == 0) {
-      // the launch's grid (launch_variant's rule for the tile shape)
-      int bx = rp->block_x, by = rp->block_y;
-      if (bx <= 0 || by <= 0 || bx * by != 128) { bx = 16; by = 8; }
-      if ((rc = ensure_tile_order(ctx, cam, rp->width, rp->height, bx, by, s, &p.tile_order)) != ST_OK) return rc;
+      if ((rc = ensure_tile_order(ctx, cam, rp->width, rp->height, tile_x, tile_y, s, &p.tile_order)) != ST_OK)
+        return rc;
     }
-    ST_CUDA(st::launch_trace(v, p, rp->block_x, rp->block_y, ctx->num_sms, s));
+    ST_CUDA(st::launch_trace(v, p, rp->block_x, rp->block_y, ctx->num_sms, ps));
     ++launches;
     return ST_OK;
   };
-  for (size_t k = 0; k < passes.size(); ++k)
-    if ((rc = run_pass(passes[k], k == 0)) != ST_OK) return rc;
+  // A pass ends on the few rays that wind longest, and a small frame is nothing
+  // else, so plain passes run side by side: the first onto the frame, the others
+  // on streams and buffers of their own, added in their order.  Four passes of
+  // 961x541 (Kerr disc) 24.0 -> 22.9 ms, of 96x54 3.57 -> 1.11 ms.
+  const bool beside = passes.size() > 1 && v.sched == ST_SCHED_PIXEL && !rp->surrogate && !depth && refine == 1 &&
+                      !p.defer_state && npix <= PASS_PIXELS;
+  if (beside) {
+    const int lanes = (int)std::min<size_t>(PASS_LANES, passes.size() - 1);
+    if ((rc = ensure_pass_lanes(ctx, npix, lanes)) != ST_OK) return rc;
+    p.beside = lanes + 1;
+    const auto all = [&]() -> int {
+      st_ray_diag* diag = p.diag;
+      // the uploads that every pass reads go before ev_open
+      const int* order = nullptr;
+      if ((rc = ensure_tile_order(ctx, cam, rp->width, rp->height, tile_x, tile_y, s, &order)) != ST_OK) return rc;
+      ST_CUDA(cudaEventRecord(ctx->ev_open, s));
+      for (int k = 0; k < (int)passes.size(); ++k) {
+        const int l = (k + lanes - 1) % lanes;
+        p.diag = k + 1 == (int)passes.size() ? diag : nullptr;  // the last pass's
+        if (k > 0) {
+          ps = ctx->pstream[l];
+          p.out = ctx->d_pass[l];
+          ST_CUDA(cudaStreamWaitEvent(ps, k <= lanes ? ctx->ev_open : ctx->ev_added[l], 0));
+        }
+        if ((rc = run_pass(passes[k], true)) != ST_OK) return rc;
+        if (k > 0) {
+          ST_CUDA(cudaEventRecord(ctx->ev_passed[l], ps));
+          ST_CUDA(cudaStreamWaitEvent(s, ctx->ev_passed[l], 0));
+          add_pass_kernel<<<(unsigned)((npix + 255) / 256), 256, 0, s>>>(ctx->d_fb, ctx->d_pass[l], npix);
+          ST_CUDA(cudaGetLastError());
+          ST_CUDA(cudaEventRecord(ctx->ev_added[l], s));
+        }
+      }
+      return ST_OK;
+    };
+    if ((rc = all()) != ST_OK) {
+      for (int l = 0; l < lanes; ++l) cudaStreamSynchronize(ctx->pstream[l]);
+      return rc;
+    }
+    p.out = ctx->d_fb;
+  } else {
+    for (size_t k = 0; k < passes.size(); ++k)
+      if ((rc = run_pass(passes[k], k == 0)) != ST_OK) return rc;
+  }
   if (refine > 1) {
     // the flagged box (+ margin), re-rendered refine - 1 more times with fresh
     // strata, then renormalised (src/metal.jl:2189-2240)
@@ -1484,6 +1563,13 @@ void st_context_destroy(st_context* ctx) {
   if (ctx->ev_coarse) cudaEventDestroy(ctx->ev_coarse);
   if (ctx->ev_fine) cudaEventDestroy(ctx->ev_fine);
   if (ctx->side) cudaStreamDestroy(ctx->side);
+  for (int l = 0; l < PASS_LANES; ++l) {
+    cudaFree(ctx->d_pass[l]);
+    if (ctx->ev_passed[l]) cudaEventDestroy(ctx->ev_passed[l]);
+    if (ctx->ev_added[l]) cudaEventDestroy(ctx->ev_added[l]);
+    if (ctx->pstream[l]) cudaStreamDestroy(ctx->pstream[l]);
+  }
+  if (ctx->ev_open) cudaEventDestroy(ctx->ev_open);
   if (ctx->ev_pass) cudaEventDestroy(ctx->ev_pass);
   if (ctx->ev_layer) cudaEventDestroy(ctx->ev_layer);
   if (ctx->lstream) cudaStreamDestroy(ctx->lstream);

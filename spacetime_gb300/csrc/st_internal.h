@@ -55,6 +55,7 @@ struct TraceParams {
   int jseed;
   float weight;
   int first_pass;            // 1: assign instead of accumulate
+  int beside;                // launches of this size side by side (0: this one alone)
   // spacetime and integration
   double M, a, rkill2;
   double r_escape, tspan;

@@ -229,14 +229,15 @@ __global__ void __launch_bounds__(32 * (1 + SPLIT_SHADERS)) trace_split_kernel(c
   flush_counters(p, steps, 0, gas, rays);
 }
 
-// The rule: whole FP32 gas frames in one launch of the pixel schedule with so few
-// rays that a step's latency and not its instructions are the frame's time.  The
+// The rule: whole FP32 gas frames of the pixel schedule with so few rays in flight
+// that a step's latency and not its instructions are the frame's time.  The
 // line (ms, Kerr / Schwarzschild, pixel kernel -> this): 320x180 2.60 / 1.99 -> 2.35 / 1.74,
 // 400x225 3.37 / 2.12 -> 3.25 / 2.59, 480x270 3.68 / 2.40 -> about 4.5 / 3.1.
 constexpr long long SPLIT_RAYS = 65536;
 inline bool split_takes(const Variant& v, const TraceParams& p) {
   return v.vol && v.sem == ST_SEM_DRAFT && v.sched == ST_SCHED_PIXEL && p.order == 4 && p.nb == 0 && !p.layer &&
-         !p.pix_list && !p.frames && p.box_cols <= 0 && (long long)p.width * p.height <= SPLIT_RAYS;
+         !p.pix_list && !p.frames && p.box_cols <= 0 &&
+         (long long)p.width * p.height * (p.beside > 1 ? p.beside : 1) <= SPLIT_RAYS;
 }
 inline cudaError_t launch_split(const Variant& v, const TraceParams& p, cudaStream_t s) {
   const dim3 grid((p.width + 7) / 8, (p.height + 3) / 4);
