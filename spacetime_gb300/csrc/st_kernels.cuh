@@ -139,19 +139,25 @@ __global__ void __launch_bounds__(128, ST_MINB) trace_resume_kernel(const __grid
   flush_counters(p, steps, f64, gas, rays);
 }
 
-// Persistent schedule: each warp pulls rays from a device queue; a lane whose
-// ray retires is refilled at the next chunk boundary (warp-ballot refill), so
-// short escaping rays do not idle lanes while photon-ring rays run on.  Queue
-// indices are ordered in 8x4 pixel tiles.  A warp takes the queue in windows of
-// refill_window consecutive indices (whole tiles: a strip of neighbouring
-// tiles) and refills its lanes from its own window before it takes the next,
-// so a refilled lane traces a neighbour of the rays still running beside it
-// (refill_window = 32: every refill from the global queue, as one tile).
+// Persistent schedule: each warp pulls rays from a device queue.  Queue indices
+// are ordered in 8x4 pixel tiles (tile_order: those of a single frame centre
+// first).  The float precisions take a tile when the last ray of the one before
+// has ended: refilled one by one, a warp's lanes drift apart, and with guard
+// steps, gas samples and disc crossings at different times nearly every step
+// runs some lane's (16 guarded 640x360 frames 71 -> 61.5 ms, 1080p FP32 Kerr gas
+// 38.8 -> 36.4).  The all-double kernels, whose step costs its warp the same
+// whatever its lanes do, refill a lane whose ray retires at the next chunk
+// boundary (warp ballot); a warp takes the queue in windows of refill_window
+// consecutive indices (whole tiles: a strip of neighbouring tiles) and refills
+// from its own window before it takes the next, so a refilled lane traces a
+// neighbour of the rays still running beside it (refill_window = 32: every
+// refill from the global queue, as one tile).
 // The outer loop is bounded by budget_iters; on exhaustion the kernel records
 // ST_EBUDGET in the status counter and returns.
 template <int PREC, int KERR, int VOL, int SEM>
 __global__ void __launch_bounds__(128, ST_MINB) trace_persistent_kernel(const __grid_constant__ TraceParams p) {
   using R = typename RealOf<PREC>::T;
+  constexpr bool WHOLE = PREC != ST_PREC_FP64;
   const unsigned FULL = 0xffffffffu;
   const int lane = (threadIdx.y * blockDim.x + threadIdx.x) & 31;
   const int tiles_x = (p.width + 7) >> 3;
@@ -166,7 +172,7 @@ __global__ void __launch_bounds__(128, ST_MINB) trace_persistent_kernel(const __
   unsigned w_next = 0, w_end = 0;  // this warp's window of the queue (warp-uniform)
   for (long long it = 0; it < p.budget_iters; ++it) {
     const unsigned idle = __ballot_sync(FULL, !active);
-    if (idle && !exhausted) {
+    if ((WHOLE ? idle == FULL : idle != 0) && !exhausted) {
       const unsigned need = (unsigned)__popc(idle);
       const unsigned rank = __popc(idle & ((1u << lane) - 1u));
       unsigned idx = 0xffffffffu;
@@ -192,7 +198,7 @@ __global__ void __launch_bounds__(128, ST_MINB) trace_persistent_kernel(const __
         if (idx < nr) {
           const int frame = (int)idx / per_frame;
           const int w = (int)idx - frame * per_frame;
-          const int tile = w >> 5, within = w & 31;
+          const int tile = p.tile_order ? __ldg(p.tile_order + (w >> 5)) : w >> 5, within = w & 31;
           const int ti = tile % tiles_x, tj = tile / tiles_x;
           const int i = ti * 8 + (within & 7), j = tj * 4 + (within >> 3);
           if (i < p.width && j < p.height) {
