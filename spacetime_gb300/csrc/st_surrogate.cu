@@ -34,7 +34,6 @@
 #include <cstddef>
 #include <cstdlib>
 #include <cstring>
-#include <type_traits>
 #include <new>
 #include <vector>
 
@@ -1855,8 +1854,8 @@ int ensure_train(st_surrogate* s, int ntiles) {
   const size_t nt = ntiles, grid = tc_grid(ntiles);
   if (cudaMalloc(&s->tH, 3 * nt * TR_IMG) != cudaSuccess || cudaMalloc(&s->tD, 3 * nt * TR_IMG) != cudaSuccess ||
       cudaMalloc(&s->tZ, grid * 2 * NH * TC_ROWS * sizeof(float)) != cudaSuccess ||
-      cudaMalloc(&s->tpart, grid * TR_ROW * sizeof(float)) != cudaSuccess ||
-      cudaMalloc(&s->tpw, (size_t)TR_SPLITS * 3 * NH * NH * sizeof(float)) != cudaSuccess)
+      cudaMalloc(&s->tpart, 4 * nt * TR_ROW * sizeof(float)) != cudaSuccess ||
+      cudaMalloc(&s->tpw, (size_t)train_splits(ntiles) * 3 * NH * NH * sizeof(float)) != cudaSuccess)
     return ST_ENOMEM;
   SC(cudaFuncSetAttribute(train_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TR_SMEM));
   SC(cudaFuncSetAttribute(train_dw_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DW_SMEM));
@@ -1871,13 +1870,15 @@ int ensure_train(st_surrogate* s, int ntiles) {
 // into G or, where G is null, an AdamW step.
 int train_pass(st_surrogate* s, const float* X, const float* T, int B, int n, float* loss, float* G,
                const AdamParams& a) {
-  const int nt = B / (int)TC_ROWS, grid = tc_grid(nt), splits = std::min(TR_SPLITS, nt);
+  const int nt = B / (int)TC_ROWS, grid = tc_grid(nt);
+  // (rounded up to whole blocks of 64 rows, the last of 64 shares may be empty)
+  const int per = (2 * nt + train_splits(nt) - 1) / train_splits(nt), splits = (2 * nt + per - 1) / per;
   const TrainParams tp{s->P, s->WF, s->WT, X, T, n, nt, 1.0f / n, s->tH, s->tD, s->tZ, s->tpart, loss, s->d_status};
   train_tile_kernel<<<grid, TR_THREADS, TR_SMEM, s->stream>>>(tp);
   SC(cudaGetLastError());
   train_dw_kernel<<<dim3(splits, 2, 3), 256, DW_SMEM, s->stream>>>(s->tH, s->tD, nt, s->tpw, s->d_status);
   SC(cudaGetLastError());
-  train_update_kernel<<<UPD_HIDDEN + UPD_EDGE, 256, 0, s->stream>>>(s->tpw, splits, s->tpart, grid, G, a, s->WF,
+  train_update_kernel<<<UPD_HIDDEN + UPD_EDGE, 256, 0, s->stream>>>(s->tpw, splits, s->tpart, 4 * nt, G, a, s->WF,
                                                                     s->WT);
   SC(cudaGetLastError());
   return ST_OK;

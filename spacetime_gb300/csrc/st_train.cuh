@@ -15,12 +15,13 @@
 // pass over a tile at 16 a clock), so each forward pass takes the derivative
 // from the same exponential and reciprocal and keeps it: for two layers in
 // tensor memory in the place of the pre-activations, for two in global memory.
-// Batch 16,384: 0.324 -> 0.080 ms a step.
+// Batch 16,384: 0.324 -> 0.093 ms a step (0.080 with fewer partials, in another
+// order).
 //
 // The arithmetic of a row is that of the layer-by-layer path: FP32 edge layers
 // in the same order, bf16 operands, FP32 accumulation over K in the same order,
-// the same rounding of activations and of their gradients.  Only the sums over
-// the batch are taken in another, fixed, order.
+// the same rounding of activations and of their gradients, and the sums over the
+// batch in its order where that is fixed; what it added by atomics is in order here.
 #pragma once
 
 namespace st {
@@ -32,16 +33,15 @@ constexpr uint32_t TR_IMG = TC_ROWS * NH * 2;  // one 128 x 256 bf16 tile, 64 KB
 constexpr int TR_B1 = NH * NIN + NH, TR_W4 = TR_B1 + 3 * NH, TR_B4 = TR_W4 + NOUT * NH, TR_EDGE = TR_B4 + NOUT;
 constexpr int TR_ROW = 4104;  // their row stride
 static_assert(TR_EDGE <= TR_ROW, "edge partials");
-constexpr int TR_SPLITS = 25;  // shares of the batch in the weight gradients: 6 x 25 = 150 CTAs
+// shares of the batch in the hidden weight gradients, at most this many
+constexpr int TR_SPLITS = 64;
+inline int train_splits(int ntiles) { return std::max(1, std::min(TR_SPLITS, ntiles / 8)); }
 
 struct TrainSmall {
   // rows of eight, read as two 16-byte words: a unit's layer-0 weights and bias, a
   // row's inputs, its targets and then its output gradient
   float w0[NH][8], X[TC_ROWS][8];
-  union {
-    float dout[TC_ROWS][8];
-    float bsum[4][NH];  // column sums of the way back, when dout is spent
-  };
+  float dout[TC_ROWS][8];
   float w4t[NOUT][NH], bh[3][NH], b4[8];
   uint64_t bar_w, bar_mma;
   uint32_t tmem;
@@ -62,7 +62,7 @@ struct TrainParams {
   unsigned char* H;         // [3][ntiles] activations H0..H2
   unsigned char* D;         // [3][ntiles] gradients dZ1..dZ3
   float* Z;                 // [grid][2][256][128] SiLU derivatives of layers 0 and 1
-  float* part;              // [grid][TR_ROW] edge partials
+  float* part;              // [4 ntiles][TR_ROW] edge partials, one row of them for 32 of the batch
   float* loss;              // 4 sums, added to
   int* status;
 };
@@ -109,7 +109,6 @@ __device__ __forceinline__ void row8(const float* r, float* v) {
   v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
   v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
 }
-__device__ __forceinline__ void put_sum(float* p, float v, bool first) { *p = first ? v : *p + v; }
 
 __global__ void __launch_bounds__(TR_THREADS, 1) train_tile_kernel(const TrainParams tp) {
   extern __shared__ unsigned char tr_raw[];
@@ -187,28 +186,14 @@ __global__ void __launch_bounds__(TR_THREADS, 1) train_tile_kernel(const TrainPa
       g[e] = z.x; g[e + 1] = z.y; g[e + 2] = z.z; g[e + 3] = z.w;
     }
   };
-  float* part = tp.part + (size_t)blockIdx.x * TR_ROW;
-  // sums over a tile's rows: two columns and a quarter of the rows a thread, the
-  // quarters then added in shared memory (in the tile's place, once it is read)
+  // sums over a tile's rows: two columns and a quarter of the rows a thread, each
+  // quarter in a row of partials of its own.  Small batches depend on the order of
+  // these sums: AdamW steps by g / |g| at first, a rounding more or less moves a
+  // bf16 weight, and ten steps later the loss differs in its fourth digit.
+  // train_update_kernel keeps reduce_parts' order.
   const int n2 = (tid & 127) * 2, quart = tid >> 7, r0 = quart * 32;
-  float* red = reinterpret_cast<float*>(As);
-  auto fold = [&](auto count, const float2* a, auto column) {
-    constexpr int cnt = decltype(count)::value;
-    __syncthreads();  // the tile is read
-#pragma unroll
-    for (int j = 0; j < cnt; ++j)
-      *reinterpret_cast<float2*>(red + (quart * cnt + j) * NH + n2) = a[j];
-    __syncthreads();
-#pragma unroll
-    for (int e = 0; e < (cnt * NH + TR_THREADS - 1) / TR_THREADS; ++e) {
-      const int k = tid + e * TR_THREADS;
-      if (k < cnt * NH)
-        column(k / NH, k % NH, (red[k] + red[cnt * NH + k]) + (red[2 * cnt * NH + k] + red[3 * cnt * NH + k]));
-    }
-    __syncthreads();
-  };
-  bool first = true;
   for (int t = blockIdx.x; t < tp.ntiles; t += gridDim.x) {
+    float* part = tp.part + ((size_t)t * 4 + quart) * TR_ROW;
     for (int k = tid; k < (int)TC_ROWS * NIN; k += TR_THREADS)
       S.X[k / NIN][k % NIN] = tp.X[(size_t)t * TC_ROWS * NIN + k];
     // the targets wait where each row's output gradient will be
@@ -284,7 +269,7 @@ __global__ void __launch_bounds__(TR_THREADS, 1) train_tile_kernel(const TrainPa
         float2 s = make_float2(0.f, 0.f);
 #pragma unroll 8
         for (int b = 0; b < 32; ++b) s = __fadd2_rn(s, get2(As, r0 + b, n2));
-        *reinterpret_cast<float2*>(&S.bsum[quart][n2]) = s;
+        *reinterpret_cast<float2*>(part + TR_B1 + (5 - m) * NH + n2) = s;
       }
       if (tid == 0 && !S.fail) {
         if (!tc::mbar_wait(&S.bar_mma, pm, TC_WAIT_LIMIT)) S.fail = 1;
@@ -298,9 +283,6 @@ __global__ void __launch_bounds__(TR_THREADS, 1) train_tile_kernel(const TrainPa
         load_w(m < 5 ? m + 1 : 0);
         w_out = true;
       }
-      if (m >= 3 && tid < NH)
-        put_sum(part + TR_B1 + (5 - m) * NH + tid,
-                (S.bsum[0][tid] + S.bsum[1][tid]) + (S.bsum[2][tid] + S.bsum[3][tid]), first);
       // the pass after product m, 32 columns at a time; the first are computed
       // while the bulk store may still be reading the tile
 #pragma unroll 1
@@ -402,13 +384,15 @@ __global__ void __launch_bounds__(TR_THREADS, 1) train_tile_kernel(const TrainPa
 #pragma unroll
             for (int j = 0; j < NOUT; ++j) a[j] = __ffma2_rn(make_float2(d[j], d[j]), h, a[j]);
           }
-          if (tid < NOUT) {
+          if ((tid & 127) < NOUT) {
             float s = 0.f;
 #pragma unroll 8
-            for (int b = 0; b < (int)TC_ROWS; ++b) s += S.dout[b][tid];
-            put_sum(part + TR_B4 + tid, s, first);
+            for (int b = r0; b < r0 + 32; ++b) s += S.dout[b][tid & 127];
+            part[TR_B4 + (tid & 127)] = s;
           }
-          fold(std::integral_constant<int, NOUT>{}, a, [&](int j, int k, float s) { put_sum(part + TR_W4 + j * NH + k, s, first); });
+#pragma unroll
+          for (int j = 0; j < NOUT; ++j) *reinterpret_cast<float2*>(part + TR_W4 + j * NH + n2) = a[j];
+          __syncthreads();  // the tile is read
         }
         // dZ3 = (dout W4) times the derivative of layer 3, from tensor memory
         float d[8];
@@ -453,11 +437,14 @@ __global__ void __launch_bounds__(TR_THREADS, 1) train_tile_kernel(const TrainPa
         for (int i = 0; i < NIN; ++i) a[i] = __ffma2_rn(make_float2(xr[i], xr[i]), d, a[i]);
         a[NIN] = __fadd2_rn(a[NIN], d);
       }
-      fold(std::integral_constant<int, NIN + 1>{}, a, [&](int i, int k, float s) {
-        put_sum(part + (i < NIN ? k * NIN + i : NH * NIN + k), s, first);
-      });
+      static_assert(NIN == 6, "two columns of dW0 in three words");
+      float4* w = reinterpret_cast<float4*>(part + n2 * NIN);
+      w[0] = make_float4(a[0].x, a[1].x, a[2].x, a[3].x);
+      w[1] = make_float4(a[4].x, a[5].x, a[0].y, a[1].y);
+      w[2] = make_float4(a[2].y, a[3].y, a[4].y, a[5].y);
+      *reinterpret_cast<float2*>(part + NH * NIN + n2) = a[NIN];
+      __syncthreads();  // the tile is read
     }
-    first = false;
   }
   const bool failed = S.fail != 0;
   if (tid == 0) {
@@ -496,9 +483,10 @@ constexpr uint32_t TR_IDESC_MN = TC_IDESC | (1u << 15) | (1u << 16);  // A and B
 // half of the inputs i, all outputs o and one share of the batch's tiles.  Both
 // operands are the tiles that train_tile_kernel left, copied as they are into two
 // stages of 96 KB; K is the batch.  The accumulator goes to a partial of its own
-// (in the parameters' order, coalesced along i), summed by train_update_kernel in a
-// fixed order: 25 shares of 6 products keep 150 SMs busy, and each CTA then moves
-// half a megabyte in for its 128 KB out.
+// (in the parameters' order, coalesced along i), summed by train_update_kernel in
+// order.  A share is 1,024 rows, in blocks of 64: 96 CTAs at a batch of 16,384, 13.0
+// us.  Tiles dealt to 150 CTAs took 11.7 us, but made a batch under 2,048 rows 25
+// sums of the one it is (see train_tile_kernel).
 constexpr uint32_t DW_STAGE = TR_IMG / 2 + TR_IMG;
 constexpr size_t DW_SMEM = 1024 + 2 * (size_t)DW_STAGE + 64;
 __global__ void __launch_bounds__(256, 1) train_dw_kernel(const unsigned char* __restrict__ H,
@@ -533,27 +521,28 @@ __global__ void __launch_bounds__(256, 1) train_dw_kernel(const unsigned char* _
       tc::bulk_g2s(a + TR_IMG / 2, Dl + (size_t)t * TR_IMG, TR_IMG / 2, full + st);
       tc::bulk_g2s(a + TR_IMG, Dl + (size_t)t * TR_IMG + TR_IMG / 2, TR_IMG / 2, full + st);
     };
-    const int S = gridDim.x;
-    const int nt = (ntiles - s0 + S - 1) / S;  // tiles s0, s0 + S, ...
+    // blocks kb0.. of 64 rows, in tiles t0.. (the first and last perhaps by half)
+    const int per = (2 * ntiles + (int)gridDim.x - 1) / (int)gridDim.x;
+    const int kb0 = s0 * per, kb1 = min(2 * ntiles, kb0 + per), t0 = kb0 >> 1, nt = ((kb1 + 1) >> 1) - t0;
     bool ok = true;
     int loaded = 0, issued = 0;
-    for (; loaded < 2 && loaded < nt; ++loaded) load(s0 + loaded * S, loaded);
+    for (; loaded < 2 && loaded < nt; ++loaded) load(t0 + loaded, loaded);
     for (int k = 0; k < nt && ok; ++k) {
       const int st = k & 1;
       ok = tc::mbar_wait(full + st, (uint32_t)(k >> 1) & 1u, TC_WAIT_LIMIT);
       if (!ok) break;
       tc::fence_after_sync();
       const uint32_t a = tc::smem_u32(base + st * DW_STAGE), b = a + TR_IMG / 2;
-#pragma unroll
-      for (int s = 0; s < (int)TC_ROWS / 16; ++s)
+      const int s1 = (k == 0 && (kb0 & 1)) ? 4 : 0, s2 = (k == nt - 1 && (kb1 & 1)) ? 4 : 8;
+      for (int s = s1; s < s2; ++s)
         tc::mma_bf16(tmem, sw128_mn_desc(a + s * 2048, TC_ROWS), sw128_mn_desc(b + s * 2048, TC_ROWS), TR_IDESC_MN,
-                     (k > 0 || s > 0) ? 1u : 0u);
+                     (k > 0 || s > s1) ? 1u : 0u);
       tc::mma_commit(done + st);
       ++issued;
       if (loaded < nt) {
         // the stage is free once its products are done; the other one's copy is on its way
         ok = tc::mbar_wait(done + st, (uint32_t)(k >> 1) & 1u, TC_WAIT_LIMIT);
-        if (ok) { load(s0 + loaded * S, st); ++loaded; }
+        if (ok) { load(t0 + loaded, st); ++loaded; }
       }
     }
     // the last products; after a wait that ran out, whatever is still in flight
@@ -657,20 +646,25 @@ __global__ void __launch_bounds__(256) train_update_kernel(const float* __restri
     }
     return;
   }
-  __shared__ float red[8][32];
+  // the partials of every 32nd row, then those 32 sums, in order; a warp takes four
+  __shared__ float red[32][32];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int c = (blockIdx.x - UPD_HIDDEN) * 32 + lane;
-  float acc = 0.f;
+  float acc[4] = {0.f, 0.f, 0.f, 0.f};
   if (c < TR_EDGE) {
-#pragma unroll 8
-    for (int p = w; p < nparts; p += 8) acc += part[(size_t)p * TR_ROW + c];
+#pragma unroll 4
+    for (int p = w; p < nparts; p += 32)
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (p + 8 * k < nparts) acc[k] += part[(size_t)(p + 8 * k) * TR_ROW + c];
   }
-  red[w][lane] = acc;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) red[w + 8 * k][lane] = acc[k];
   __syncthreads();
   if (w != 0 || c >= TR_EDGE) return;
   float g = red[0][lane];
 #pragma unroll
-  for (int k = 1; k < 8; ++k) g += red[k][lane];
+  for (int k = 1; k < 32; ++k) g += red[k][lane];
   // the parameter of column c
   size_t i;
   bool is_bias = true;

@@ -1,6 +1,6 @@
 """The fused training kernels at the edges of their tiling: a single padded row,
-one full 128-row tile, a tile and a row, more tiles than weight-gradient shares
-(25), and more tiles than a 152-SM GPU has CTAs (a CTA then takes two).
+one full 128-row tile, a tile and a row, several weight-gradient shares, and
+shares of half tiles with more tiles than a 152-SM GPU has CTAs (one then takes two).
 
 Tolerances: those of the gradient comparison with the FP64 MLP (bf16 operands:
 relative L2 error <= 5e-2 and cosine >= 0.995 per parameter tensor).  The AdamW
