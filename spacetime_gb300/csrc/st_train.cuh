@@ -15,7 +15,7 @@
 // pass over a tile at 16 a clock), so each forward pass takes the derivative
 // from the same exponential and reciprocal and keeps it: for two layers in
 // tensor memory in the place of the pre-activations, for two in global memory.
-// Batch 16,384: 0.324 -> 0.093 ms a step (0.080 with fewer partials, in another
+// Batch 16,384: 0.324 -> 0.086 ms a step (0.080 with fewer partials, in another
 // order).
 //
 // The arithmetic of a row is that of the layer-by-layer path: FP32 edge layers
@@ -190,7 +190,9 @@ __global__ void __launch_bounds__(TR_THREADS, 1) train_tile_kernel(const TrainPa
   // quarter in a row of partials of its own.  Small batches depend on the order of
   // these sums: AdamW steps by g / |g| at first, a rounding more or less moves a
   // bf16 weight, and ten steps later the loss differs in its fourth digit.
-  // train_update_kernel keeps reduce_parts' order.
+  // train_update_kernel keeps reduce_parts' order.  (Their loops over rows are
+  // unrolled by four: by eight they spill, and there is next to no L1 beside the
+  // shared memory, 59.0 -> 51.9 us.)
   const int n2 = (tid & 127) * 2, quart = tid >> 7, r0 = quart * 32;
   for (int t = blockIdx.x; t < tp.ntiles; t += gridDim.x) {
     float* part = tp.part + ((size_t)t * 4 + quart) * TR_ROW;
@@ -376,7 +378,7 @@ __global__ void __launch_bounds__(TR_THREADS, 1) train_tile_kernel(const TrainPa
           float2 a[NOUT];
 #pragma unroll
           for (int j = 0; j < NOUT; ++j) a[j] = make_float2(0.f, 0.f);
-#pragma unroll 8
+#pragma unroll 4
           for (int b = r0; b < r0 + 32; ++b) {
             const float2 h = get2(As, b, n2);
             float d[8];
@@ -428,7 +430,7 @@ __global__ void __launch_bounds__(TR_THREADS, 1) train_tile_kernel(const TrainPa
       float2 a[NIN + 1];
 #pragma unroll
       for (int i = 0; i <= NIN; ++i) a[i] = make_float2(0.f, 0.f);
-#pragma unroll 8
+#pragma unroll 4
       for (int b = r0; b < r0 + 32; ++b) {
         const float2 d = get2(As, b, n2);
         float xr[8];
