@@ -1866,6 +1866,23 @@ int ensure_train(st_surrogate* s, int ntiles) {
   return ST_OK;
 }
 
+// A launch that may start before the kernel ahead of it in the stream has ended
+// (wait_for_previous in st_train.cuh).
+template <class... P, class... A>
+cudaError_t launch_dependent(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t stream, A... args) {
+  cudaLaunchAttribute early{};
+  early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  early.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t c{};
+  c.gridDim = grid;
+  c.blockDim = dim3(threads);
+  c.dynamicSmemBytes = smem;
+  c.stream = stream;
+  c.attrs = &early;
+  c.numAttrs = 1;
+  return cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...);
+}
+
 // Loss sums (added to loss[4]) and gradient of B padded rows, n of which count,
 // into G or, where G is null, an AdamW step.
 int train_pass(st_surrogate* s, const float* X, const float* T, int B, int n, float* loss, float* G,
@@ -1874,13 +1891,11 @@ int train_pass(st_surrogate* s, const float* X, const float* T, int B, int n, fl
   // (rounded up to whole blocks of 64 rows, the last of 64 shares may be empty)
   const int per = (2 * nt + train_splits(nt) - 1) / train_splits(nt), splits = (2 * nt + per - 1) / per;
   const TrainParams tp{s->P, s->WF, s->WT, X, T, n, nt, 1.0f / n, s->tH, s->tD, s->tZ, s->tpart, loss, s->d_status};
-  train_tile_kernel<<<grid, TR_THREADS, TR_SMEM, s->stream>>>(tp);
-  SC(cudaGetLastError());
-  train_dw_kernel<<<dim3(splits, 2, 3), 256, DW_SMEM, s->stream>>>(s->tH, s->tD, nt, s->tpw, s->d_status);
-  SC(cudaGetLastError());
-  train_update_kernel<<<UPD_HIDDEN + UPD_EDGE, 256, 0, s->stream>>>(s->tpw, splits, s->tpart, 4 * nt, G, a, s->WF,
-                                                                    s->WT);
-  SC(cudaGetLastError());
+  SC(launch_dependent(train_tile_kernel, grid, TR_THREADS, TR_SMEM, s->stream, tp));
+  SC(launch_dependent(train_dw_kernel, dim3(splits, 2, 3), 256, DW_SMEM, s->stream, s->tH, s->tD, nt, s->tpw,
+                      s->d_status));
+  SC(launch_dependent(train_update_kernel, UPD_HIDDEN + UPD_EDGE, 256, 0, s->stream, s->tpw, splits, s->tpart, 4 * nt,
+                      G, a, s->WF, s->WT));
   return ST_OK;
 }
 
