@@ -21,11 +21,12 @@ LIB = os.environ.get("SPACETIME_GB300_LIB", os.path.join(HERE, "libspacetime_gb3
 FAST = os.environ.get("ST_FASTMATH", "1") == "1"
 MINB_FP32 = os.environ.get("ST_MINB_FP32", "7")
 MINB_FP32G = os.environ.get("ST_MINB_FP32G", "5")
+MINB_FP32G_KERR = os.environ.get("ST_MINB_FP32G_KERR", "4")
 MINB_FP64 = os.environ.get("ST_MINB_FP64", "1")
 MINB_PAIRS = os.environ.get("ST_MINB_PAIRS", "12")
 UNIT_FLAGS = {
     "st_trace_fp32.cu": (["--use_fast_math"] if FAST else []) + [f"-DST_MINB={MINB_FP32}"],
-    "st_trace_fp32_guarded.cu": (["--use_fast_math"] if FAST else []) + [f"-DST_MINB={MINB_FP32G}"],
+    "st_trace_fp32_guarded.cu": (["--use_fast_math"] if FAST else []) + [f"-DST_MINB={MINB_FP32G}", f"-DST_MINB_KERR={MINB_FP32G_KERR}"],
     "st_trace_fp64.cu": [f"-DST_MINB={MINB_FP64}"],
     "st_trace_pairs.cu": [f"-DST_PAIR_MINB={MINB_PAIRS}"],
     # the fluid solver rounds every float operation as written (no contraction)

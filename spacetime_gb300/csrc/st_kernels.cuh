@@ -11,6 +11,11 @@
 #ifndef ST_MINB
 #define ST_MINB 1
 #endif
+// That of the Kerr pixel kernels without gas.  Guarded: 4, with 128 registers (the
+// figures are at guard_step in st_trace.cuh); the others keep 5.
+#ifndef ST_MINB_KERR
+#define ST_MINB_KERR ST_MINB
+#endif
 // The adaptive Tsit5 modes (order 45 / 46) hold more state per ray; they keep
 // the budget of at most 5 blocks.
 #ifndef ST_MINB_ADAPTIVE
@@ -42,7 +47,7 @@ __device__ __forceinline__ void flush_counters(const TraceParams& p, unsigned lo
 // One thread per pixel over a 2-D grid of tiles (blockDim.x * blockDim.y a
 // multiple of 32; threads are linearised so a warp covers a compact tile).
 template <int PREC, int KERR, int VOL, int SEM, int ORD = 4, int DEPTH = 0, int DEFER = 0>
-__global__ void __launch_bounds__(128, ORD == 4 ? ST_MINB : ST_MINB_ADAPTIVE) trace_pixel_kernel(const __grid_constant__ TraceParams p) {
+__global__ void __launch_bounds__(128, ORD != 4 ? ST_MINB_ADAPTIVE : KERR && !VOL ? ST_MINB_KERR : ST_MINB) trace_pixel_kernel(const __grid_constant__ TraceParams p) {
   using R = typename RealOf<PREC>::T;
   if (p.lut_stage) {
     // the blackbody table into shared memory, once per block (16 KiB for the
