@@ -455,13 +455,14 @@ cudaError_t launch_pairs(const TraceParams& p, int bx, int by, cudaStream_t s) {
 
 // The rule: RK4 frames of the pixel schedule whose lengths and times keep every
 // intermediate of the right-hand side (up to r^4 and 1 / r^2, with 48 bits
-// below) far inside a float's exponent.  Everything else -- the adaptive
+// below) far inside a float's exponent, and whose gas absorbs (with a negative
+// opacity e^-tau grows beyond a float's range).  Everything else -- the adaptive
 // integrators, the layered engine's layer, depth buckets, the persistent queue
 // and scenes in other units -- stays on the all-double kernels.
 bool pairs_take(const Variant& v, const TraceParams& p) {
   return v.prec == ST_PREC_FP64 && v.sched == ST_SCHED_PIXEL && p.order == 4 && p.nb == 0 && !p.layer &&
          p.M >= 1.0 / 64 && p.M <= 64.0 && p.r_max > 0.0 && p.r_max <= 1e5 && p.dt >= 1e-5 && p.dt <= 100.0 &&
-         p.tspan <= 1e7;
+         p.tspan <= 1e7 && (!p.vol_on || p.opac >= 0.0);
 }
 
 cudaError_t launch_trace_pairs(const Variant& v, const TraceParams& p, int bx, int by, cudaStream_t s) {
