@@ -519,6 +519,14 @@ ST_DF void rk4_six(const df2* y, df2 pt, const Hole& H, df2 h, df2* inc) {
   for (int k = 0; k < 6; ++k) inc[k] = mul(h6, s[k]);
 }
 
+// x + y with one rounding of x's low part, for |y| < |x|: half an ulp of it where
+// add is off by one or two.  For a state that is added to at every step, whose
+// rounding is then all that a guarded ray is off by.
+ST_DF df2 add_rn(df2 x, df2 y) {
+  const df2 s = two_sum(x.hi, y.hi), u = two_sum(s.lo, x.lo), v = fast(s.hi, u.hi);
+  return fast(v.hi, fadd(v.lo, fadd(u.lo, y.lo)));
+}
+
 // ---------------------------------------------------------------------------
 // Shading.  Its results go into a float image, so its pairs are kept to about
 // 2^-40: products and sums without the last renormalisation (half the

@@ -1136,9 +1136,10 @@ __device__ __forceinline__ R tsit5_adaptive(const R* s0, R pt, R M, R a, R r, R 
 
 // The guarded path's guard step and null renormalisation, on its float-float
 // state, in the float pairs of st_df.cuh.  The state holds 48 bits whatever the
-// step is computed in: in double and in pairs the exit directions of fully
-// guarded rays are off by the same 3.2e-14 to 3.7e-14 (median over cameras and
-// spins, against 128-bit arithmetic), which is the state's own rounding.  A
+// step is computed in, so with one rounding a step (add_rn) the exit directions of
+// fully guarded rays are off by 1.9e-14 to 2.1e-14 in pairs and 1.8e-14 to 2.2e-14
+// in double (medians over directions, four spins, against 128-bit arithmetic;
+// 3.4e-14 with add's two or three roundings; tests/test_df_guard.py).  A
 // double guard step held its whole warp for about 5,900 cycles of the SM's FP64
 // pipe, and the frame ended on the rays that are guarded all the way.
 //
@@ -1149,9 +1150,9 @@ __device__ __forceinline__ R tsit5_adaptive(const R* s0, R pt, R M, R a, R r, R 
 // a 640x360 Schwarzschild disc frame issued 0.65 a cycle, plain 0.81, and the
 // Kerr step spilled its loop's registers (28 to 436 bytes; plain none).  Guards
 // at their defaults, ms, in an earlier double-float step / packed / plain:
-// Schwarzschild disc 480x270 6.5 / 7.5 / 6.4, 640x360 7.2 / 8.6 / 7.2, 1080p 22.9 /
-// 22.6 / 21.5; Kerr without matter 480x270 16.6 / 15.0 / 11.6, 1080p 41.0 / 39.1 / 37.3;
-// Kerr gas 480x270 18.8 / 17.4 / 15.0, 1080p 64.0 / 59.0 / 53.0 (134 in double).
+// Schwarzschild disc 480x270 6.5 / 7.5 / 6.5, 640x360 7.3 / 8.6 / 7.4, 1080p 22.9 /
+// 22.6 / 21.6; Kerr without matter 480x270 16.6 / 15.0 / 11.7, 1080p 41.0 / 39.1 / 37.4;
+// Kerr gas 480x270 18.8 / 17.4 / 15.1, 1080p 64.0 / 59.0 / 53.3 (134 in double).
 template <int KERR>
 __device__ __forceinline__ void guard_step(float* y, float* lo, float pt, const dfm::Hole& H, float h) {
   using namespace dfm;
@@ -1161,7 +1162,7 @@ __device__ __forceinline__ void guard_step(float* y, float* lo, float pt, const 
   rk4_six<KERR>(Y, q(pt), H, q(h), inc);
 #pragma unroll
   for (int k = 0; k < 6; ++k) {
-    const df2 v = add(Y[k], inc[k]);
+    const df2 v = add_rn(Y[k], inc[k]);
     y[k] = v.hi;
     lo[k] = v.lo;
   }
