@@ -792,7 +792,7 @@ int do_render(st_context* ctx, const st_camera* cam, const st_spacetime* stp, co
   if ((rc = ensure(&ctx->d_fb, &ctx->fb_cap, npix)) != ST_OK) return rc;
   if (host_rgb && (rc = ensure(&ctx->d_rgb, &ctx->rgb_cap, 3 * npix)) != ST_OK) return rc;
   if (host_diag && (rc = ensure(&ctx->d_diag, &ctx->diag_cap, npix)) != ST_OK) return rc;
-  p.r_max = p.r_escape;
+  p.pair_range = st::in_pair_range(p.r_escape) ? 1 : 0;
   p.out = ctx->d_fb;
   p.diag = host_diag ? ctx->d_diag : nullptr;
   p.ap_r = cam->aperture_world > 0.0 ? cam->aperture_world / 2.0 : 0.0;
@@ -1751,7 +1751,6 @@ int st_render_frames(st_context* ctx, int nframes, const st_camera* cams, const 
     fc[f].nmax = q.nmax;
     fc[f].pad = 0;
     nmax_max = std::max(nmax_max, q.nmax);
-    p.r_max = std::max(p.r_max, q.r_escape);
   }
   if ((rc = ensure(&ctx->d_frames, &ctx->frames_cap, (size_t)nframes)) != ST_OK) return rc;
   if ((rc = ensure(&ctx->d_fb, &ctx->fb_cap, npix * nframes)) != ST_OK) return rc;
@@ -1766,14 +1765,7 @@ int st_render_frames(st_context* ctx, int nframes, const st_camera* cams, const 
   p.frames = ctx->d_frames;
   p.n_frames = nframes;
   p.frame_stride = (int)npix;
-  // the frame-independent camera fields are unused with a frame table: zero
-  // them so the graph key depends only on sizes and rules
-  std::memset(p.pos, 0, sizeof p.pos);
-  std::memset(p.Ef, 0, sizeof p.Ef);
-  std::memset(p.Er, 0, sizeof p.Er);
-  std::memset(p.Eu, 0, sizeof p.Eu);
-  std::memset(p.U, 0, sizeof p.U);
-  p.r_escape = 0.0;
+  st::use_frame_table(&p, fc, nframes);
   const long long tiles = (long long)((rp->width + 7) / 8) * ((rp->height + 3) / 4);
   // the queue counts rays of whole 8x4 tiles in a 32-bit int
   if (tiles * 32 * nframes > (long long)INT_MAX) return ST_EINVAL;

@@ -165,8 +165,27 @@ struct TraceParams {
   // the same as float pairs, for the guard steps and for the FP64 frames that
   // integrate on the FP32 pipe
   dfm::Scene d;
-  double r_max;              // largest escape radius of the launch's frames (0: not known)
+  int pair_range;            // every frame's escape radius is within PAIR_R_MAX (0: not known)
 };
+
+// Escape radii to which the FP64 frames integrate in float pairs (pairs_take in
+// st_trace_pairs.cu).
+constexpr double PAIR_R_MAX = 1e5;
+inline bool in_pair_range(double r_escape) { return r_escape > 0.0 && r_escape <= PAIR_R_MAX; }
+
+// For a launch that takes its cameras from a table of n frames: its own camera's
+// fields are unused and cleared, and of the frames' radii it keeps only whether
+// they are in the pair kernel's range, so that the launch block, by which a
+// captured track is recognised, does not change as the cameras move.
+inline void use_frame_table(TraceParams* p, const FrameCam* fc, int n) {
+  for (double& v : p->pos) v = 0.0;
+  for (double* v : {p->Ef, p->Er, p->Eu, p->U})
+    for (int k = 0; k < 4; ++k) v[k] = 0.0;
+  p->r_escape = 0.0;
+  p->pair_range = 1;
+  for (int f = 0; f < n; ++f)
+    if (!in_pair_range(fc[f].r_escape)) p->pair_range = 0;
+}
 
 inline df2 host_pair(double v) {
   const float h = (float)v;

@@ -461,7 +461,7 @@ cudaError_t launch_pairs(const TraceParams& p, int bx, int by, cudaStream_t s) {
 // and scenes in other units -- stays on the all-double kernels.
 bool pairs_take(const Variant& v, const TraceParams& p) {
   return v.prec == ST_PREC_FP64 && v.sched == ST_SCHED_PIXEL && p.order == 4 && p.nb == 0 && !p.layer &&
-         p.M >= 1.0 / 64 && p.M <= 64.0 && p.r_max > 0.0 && p.r_max <= 1e5 && p.dt >= 1e-5 && p.dt <= 100.0 &&
+         p.M >= 1.0 / 64 && p.M <= 64.0 && p.pair_range && p.dt >= 1e-5 && p.dt <= 100.0 &&
          p.tspan <= 1e7 && (!p.vol_on || p.opac >= 0.0);
 }
 
