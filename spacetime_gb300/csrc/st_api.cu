@@ -381,9 +381,31 @@ int ensure(T** ptr, size_t* cap, size_t n) {
   if (*ptr) cudaFree(*ptr);
   *ptr = nullptr;
   *cap = 0;
-  if (cudaMalloc((void**)ptr, n * sizeof(T)) != cudaSuccess) return ST_ENOMEM;
+  if (cudaMalloc((void**)ptr, n * sizeof(T)) != cudaSuccess) {
+    (void)cudaGetLastError();  // not for the next launch check to find
+    return ST_ENOMEM;
+  }
   *cap = n;
   return ST_OK;
+}
+
+// The buffers that a frame's passes beside its first have left in the context:
+// given up when another buffer needs the memory.
+void drop_pass_buffers(st_context* ctx) {
+  for (int l = 0; l < PASS_LANES; ++l) {
+    cudaFree(ctx->d_pass[l]);
+    ctx->d_pass[l] = nullptr;
+    ctx->pass_cap[l] = 0;
+  }
+}
+template <class T>
+int ensure(st_context* ctx, T** ptr, size_t* cap, size_t n) {
+  int rc = ensure(ptr, cap, n);
+  if (rc == ST_ENOMEM) {
+    drop_pass_buffers(ctx);
+    rc = ensure(ptr, cap, n);
+  }
+  return rc;
 }
 
 double norm3(const double* v) { return std::sqrt(v[0] * v[0] + v[1] * v[1] + v[2] * v[2]); }
@@ -403,7 +425,7 @@ int setup_defer(st_context* ctx, TraceParams* p, const st::Variant& v, size_t nr
   const char* e = std::getenv("SPACETIME_GB300_GUARD_DEFER");
   if (!e || std::strcmp(e, "1") != 0) return ST_OK;
   if (nrays > (size_t)INT_MAX) return ST_EINVAL;
-  int rc = ensure(&ctx->d_defer, &ctx->defer_cap, nrays * st::guarded_ray_state_bytes());
+  int rc = ensure(ctx, &ctx->d_defer, &ctx->defer_cap, nrays * st::guarded_ray_state_bytes());
   if (rc != ST_OK) return rc;
   if (!ctx->d_defer_count && cudaMalloc(&ctx->d_defer_count, sizeof(unsigned)) != cudaSuccess) return ST_ENOMEM;
   p->defer_state = ctx->d_defer;
@@ -694,18 +716,20 @@ __global__ void add_pass_kernel(float4* __restrict__ fb, const float4* __restric
   fb[k] = o;
 }
 
-// Streams, events and buffers for the passes beside a frame's first.
+// Streams, events and buffers for the passes beside a frame's first: how many of
+// them there are, up to `lanes`.  Memory that is not to be had costs a lane, not
+// the frame.
 int ensure_pass_lanes(st_context* ctx, size_t npix, int lanes) {
-  if (!ctx->ev_open && cudaEventCreateWithFlags(&ctx->ev_open, cudaEventDisableTiming) != cudaSuccess) return ST_ECUDA;
-  for (int l = 0; l < lanes; ++l) {
+  const auto have = [&](int l) {
     if (!ctx->pstream[l] && cudaStreamCreateWithFlags(&ctx->pstream[l], cudaStreamNonBlocking) != cudaSuccess)
-      return ST_ECUDA;
-    for (cudaEvent_t* e : {&ctx->ev_passed[l], &ctx->ev_added[l]})
-      if (!*e && cudaEventCreateWithFlags(e, cudaEventDisableTiming) != cudaSuccess) return ST_ECUDA;
-    const int rc = ensure(&ctx->d_pass[l], &ctx->pass_cap[l], npix);
-    if (rc != ST_OK) return rc;
-  }
-  return ST_OK;
+      return false;
+    for (cudaEvent_t* e : {&ctx->ev_open, &ctx->ev_passed[l], &ctx->ev_added[l]})
+      if (!*e && cudaEventCreateWithFlags(e, cudaEventDisableTiming) != cudaSuccess) return false;
+    return ensure(&ctx->d_pass[l], &ctx->pass_cap[l], npix) == ST_OK;
+  };
+  for (int l = 0; l < lanes; ++l)
+    if (!have(l)) return l;
+  return lanes;
 }
 
 // Iteration budget of the persistent kernel's outer loop: enough for every
@@ -749,7 +773,7 @@ int ensure_tile_order(st_context* ctx, const st_camera* cam, int width, int heig
   const int cx = std::min(std::max((int)std::floor(hi / bx), 0), gx - 1);
   const int cy = std::min(std::max((int)std::floor(hj / by), 0), gy - 1);
   if (ctx->order_key[0] != gx || ctx->order_key[1] != gy || ctx->order_key[2] != cx || ctx->order_key[3] != cy) {
-    int rc = ensure(&ctx->d_order, &ctx->order_cap, (size_t)n);
+    int rc = ensure(ctx, &ctx->d_order, &ctx->order_cap, (size_t)n);
     if (rc != ST_OK) return rc;
     const int maxd = std::max(std::max(cx, gx - 1 - cx), std::max(cy, gy - 1 - cy));
     std::vector<int> start(maxd + 2, 0);
@@ -789,9 +813,9 @@ int do_render(st_context* ctx, const st_camera* cam, const st_spacetime* stp, co
   if (cudaSetDevice(ctx->device) != cudaSuccess) return ST_ECUDA;
   ctx->h2d_extra = 0;
   const size_t npix = (size_t)rp->width * rp->height;
-  if ((rc = ensure(&ctx->d_fb, &ctx->fb_cap, npix)) != ST_OK) return rc;
-  if (host_rgb && (rc = ensure(&ctx->d_rgb, &ctx->rgb_cap, 3 * npix)) != ST_OK) return rc;
-  if (host_diag && (rc = ensure(&ctx->d_diag, &ctx->diag_cap, npix)) != ST_OK) return rc;
+  if ((rc = ensure(ctx, &ctx->d_fb, &ctx->fb_cap, npix)) != ST_OK) return rc;
+  if (host_rgb && (rc = ensure(ctx, &ctx->d_rgb, &ctx->rgb_cap, 3 * npix)) != ST_OK) return rc;
+  if (host_diag && (rc = ensure(ctx, &ctx->d_diag, &ctx->diag_cap, npix)) != ST_OK) return rc;
   p.pair_range = st::in_pair_range(p.r_escape) ? 1 : 0;
   p.out = ctx->d_fb;
   p.diag = host_diag ? ctx->d_diag : nullptr;
@@ -801,7 +825,7 @@ int do_render(st_context* ctx, const st_camera* cam, const st_spacetime* stp, co
   if (rp->surrogate) {
     if (!surrogate_domain(cam, stp, &sf)) return ST_EUNSUPPORTED;
     sf.sigma_max = rp->surrogate_sigma > 0.0 ? rp->surrogate_sigma : 1e-4;
-    if ((rc = ensure(&ctx->d_list, &ctx->list_cap, npix)) != ST_OK) return rc;
+    if ((rc = ensure(ctx, &ctx->d_list, &ctx->list_cap, npix)) != ST_OK) return rc;
     if (!ctx->d_count && cudaMalloc(&ctx->d_count, sizeof(int)) != cudaSuccess) return ST_ENOMEM;
     v.sched = ST_SCHED_PIXEL;
   }
@@ -811,14 +835,14 @@ int do_render(st_context* ctx, const st_camera* cam, const st_spacetime* stp, co
     if (rp->semantics != ST_SEM_DRAFT || rp->surrogate || refine > 1) return ST_EUNSUPPORTED;
     if (p.order != 4) return ST_EUNSUPPORTED;  // render_depth_mtl integrates with RK4
     v.sched = ST_SCHED_PIXEL;                  // the bucket kernels are pixel-scheduled
-    if ((rc = ensure(&ctx->d_buckets, &ctx->buckets_cap, 3 * (size_t)depth->nb * npix)) != ST_OK) return rc;
+    if ((rc = ensure(ctx, &ctx->d_buckets, &ctx->buckets_cap, 3 * (size_t)depth->nb * npix)) != ST_OK) return rc;
     ST_CUDA(cudaMemsetAsync(ctx->d_buckets, 0, 3 * (size_t)depth->nb * npix * sizeof(float), s));
     p.nb = depth->nb;
     p.buckets = ctx->d_buckets;
   }
   if (refine > 1) {
     if (rp->semantics != ST_SEM_DRAFT || rp->surrogate) return ST_EUNSUPPORTED;
-    if ((rc = ensure(&ctx->d_stat, &ctx->stat_cap, npix)) != ST_OK) return rc;
+    if ((rc = ensure(ctx, &ctx->d_stat, &ctx->stat_cap, npix)) != ST_OK) return rc;
     if (!ctx->d_box && cudaMalloc(&ctx->d_box, 4 * sizeof(unsigned)) != cudaSuccess) return ST_ENOMEM;
     v.sched = ST_SCHED_PIXEL;  // refinement passes dispatch a box of the pixel grid
   }
@@ -894,9 +918,8 @@ int do_render(st_context* ctx, const st_camera* cam, const st_spacetime* stp, co
   // 961x541 (Kerr disc) 24.0 -> 22.9 ms, of 96x54 3.57 -> 1.11 ms.
   const bool beside = passes.size() > 1 && v.sched == ST_SCHED_PIXEL && !rp->surrogate && !depth && refine == 1 &&
                       !p.defer_state && npix <= PASS_PIXELS;
-  if (beside) {
-    const int lanes = (int)std::min<size_t>(PASS_LANES, passes.size() - 1);
-    if ((rc = ensure_pass_lanes(ctx, npix, lanes)) != ST_OK) return rc;
+  const int lanes = beside ? ensure_pass_lanes(ctx, npix, (int)std::min<size_t>(PASS_LANES, passes.size() - 1)) : 0;
+  if (lanes > 0) {
     p.beside = lanes + 1;
     const auto all = [&]() -> int {
       st_ray_diag* diag = p.diag;
@@ -1237,16 +1260,16 @@ int layered_render(st_context* ctx, const st_camera* cam, const st_spacetime* st
   if (cudaSetDevice(ctx->device) != cudaSuccess) return ST_ECUDA;
   cudaStream_t s = ctx->stream;
   const size_t npix = (size_t)rp->width * rp->height;
-  if ((rc = ensure(&ctx->d_fb, &ctx->fb_cap, npix)) != ST_OK) return rc;
-  if ((rc = ensure(&ctx->d_rgb, &ctx->rgb_cap, 3 * npix)) != ST_OK) return rc;
-  if (host_diag && (rc = ensure(&ctx->d_diag, &ctx->diag_cap, npix)) != ST_OK) return rc;
+  if ((rc = ensure(ctx, &ctx->d_fb, &ctx->fb_cap, npix)) != ST_OK) return rc;
+  if ((rc = ensure(ctx, &ctx->d_rgb, &ctx->rgb_cap, 3 * npix)) != ST_OK) return rc;
+  if (host_diag && (rc = ensure(ctx, &ctx->d_diag, &ctx->diag_cap, npix)) != ST_OK) return rc;
   const bool matter = ctx->disc_on || ctx->vol_on;
-  if (matter && (rc = ensure(&ctx->d_layer, &ctx->layer_cap, (size_t)lw * lh)) != ST_OK) return rc;
+  if (matter && (rc = ensure(ctx, &ctx->d_layer, &ctx->layer_cap, (size_t)lw * lh)) != ST_OK) return rc;
   // the ring pass (render_layered_gpu!'s ring_out / ring_rmin, src/metal.jl:3102-3118)
   const bool use_ring = matter && ring.rmin > 0.0;
   const int rw = ring.width > 0 ? ring.width : rp->width, rh = ring.height > 0 ? ring.height : rp->height;
   if (use_ring && (rw < 2 || rh < 2 || (long long)rw * rh > (1ll << 30))) return ST_EINVAL;
-  if (use_ring && (rc = ensure(&ctx->d_ring, &ctx->ring_cap, (size_t)rw * rh)) != ST_OK) return rc;
+  if (use_ring && (rc = ensure(ctx, &ctx->d_ring, &ctx->ring_cap, (size_t)rw * rh)) != ST_OK) return rc;
   if (use_ring && !ctx->lstream && cudaStreamCreateWithFlags(&ctx->lstream, cudaStreamNonBlocking) != cudaSuccess)
     return ST_ECUDA;
   for (cudaEvent_t* e : {&ctx->ev_pass, &ctx->ev_layer})
@@ -1752,9 +1775,9 @@ int st_render_frames(st_context* ctx, int nframes, const st_camera* cams, const 
     fc[f].pad = 0;
     nmax_max = std::max(nmax_max, q.nmax);
   }
-  if ((rc = ensure(&ctx->d_frames, &ctx->frames_cap, (size_t)nframes)) != ST_OK) return rc;
-  if ((rc = ensure(&ctx->d_fb, &ctx->fb_cap, npix * nframes)) != ST_OK) return rc;
-  if ((rc = ensure(&ctx->d_rgb, &ctx->rgb_cap, 3 * npix * nframes)) != ST_OK) return rc;
+  if ((rc = ensure(ctx, &ctx->d_frames, &ctx->frames_cap, (size_t)nframes)) != ST_OK) return rc;
+  if ((rc = ensure(ctx, &ctx->d_fb, &ctx->fb_cap, npix * nframes)) != ST_OK) return rc;
+  if ((rc = ensure(ctx, &ctx->d_rgb, &ctx->rgb_cap, 3 * npix * nframes)) != ST_OK) return rc;
   cudaStream_t s = ctx->stream;
   const std::vector<PassPlan> passes = plan_passes(rp, &cams[0]);
   const PassPlan& pp = passes[0];
