@@ -316,7 +316,7 @@ int st_render_depth(st_context* ctx, const st_camera* cam, const st_spacetime* s
  * A 2-D stable-fluids solver (semi-Lagrangian advection on the Keplerian
  * shear, curl-noise forcing, Jacobi pressure projection, MacCormack density
  * advection relaxed toward the disc profile) on the context volume's own
- * (log s, phi) grid; every step extrudes the surface density through the
+ * (log s, phi) grid; every call extrudes the surface density through the
  * vertical envelope exp(-z^2 / 2 H^2), H = scale_height s, into the
  * context's density texture, so the next render traces the new gas.  The
  * solver starts from the texture's midplane slice (k = (nz + 1) / 2,
@@ -338,8 +338,13 @@ void st_fluid_params_default(st_fluid_params* p);
 int st_fluid_create(st_fluid** out, st_context* ctx, const st_disc* disc, const st_fluid_params* p);
 /* nsteps steps of dt (step_sim! defaults: dt 0.05, jacobi 8, i.e.
  * 2 ceil(jacobi / 2) Jacobi sweeps), queued on the context's stream.
- * The steps of a call are one launch whatever use_graph says; ms (may be
- * NULL) receives the device time of the steps (the call then waits for them). */
+ * How they are launched does not depend on use_graph (up to 1024 steps a launch;
+ * grids that fill the GPU several times over, a few launches a step); ms (may be
+ * NULL) receives the device time of the steps (the call then waits for them).
+ * The launches' own waits are bounded.  Should one run out, the fields and the
+ * texture are not to be used: a call that waits (ms, st_fluid_state), the next step
+ * and the context's renders return ST_ECUDA, until the context is given a volume
+ * again or a new solver is created; the solver itself stays failed. */
 int st_fluid_step(st_fluid* f, double dt, int jacobi, int nsteps, int use_graph, float* ms);
 /* Host copies of the solver state ((nr, nphi) column-major; any may be NULL):
  * the velocity, the surface density, the context's density texture

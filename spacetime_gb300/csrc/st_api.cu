@@ -336,6 +336,8 @@ struct st_context {
   cudaEvent_t ev_coarse = nullptr, ev_fine = nullptr;
   cudaStream_t lstream = nullptr;  // the layer pass runs here, beside the ring pass
   cudaEvent_t ev_pass = nullptr, ev_layer = nullptr;
+  // set by a fluid solver whose steps were given up (pinned, mapped)
+  volatile int* gas_fault = nullptr;
   // the passes of a frame beside its first: a stream and a frame buffer each,
   // the pass's end and its addition to the frame
   cudaStream_t pstream[PASS_LANES] = {};
@@ -406,6 +408,13 @@ int ensure(st_context* ctx, T** ptr, size_t* cap, size_t n) {
     rc = ensure(ptr, cap, n);
   }
   return rc;
+}
+
+// A finished launch's status: its counters' word, or that the gas it sampled is a
+// fluid solver's whose steps were given up.
+int launch_status(const st_context* ctx, const unsigned long long* cnt) {
+  if (cnt[st::CNT_STATUS]) return (int)cnt[st::CNT_STATUS];
+  return ctx->vol_on && ctx->gas_fault && *ctx->gas_fault ? ST_ECUDA : ST_OK;
 }
 
 double norm3(const double* v) { return std::sqrt(v[0] * v[0] + v[1] * v[1] + v[2] * v[2]); }
@@ -1007,7 +1016,7 @@ int do_render(st_context* ctx, const st_camera* cam, const st_spacetime* stp, co
   }
   ST_CUDA(cudaStreamSynchronize(s));
   if (dev_rgba) *dev_rgba = reinterpret_cast<const float*>(ctx->d_fb);
-  const int status = cnt[st::CNT_STATUS] ? (int)cnt[st::CNT_STATUS] : ST_OK;
+  const int status = launch_status(ctx, cnt);
   if (stats) {
     float ms = 0.f;
     // a failed query must not leave an error pending for the next launch check
@@ -1154,6 +1163,26 @@ int context_volume(st_context* ctx, CtxVolume* out) {
   out->on = ctx->vol_on && ctx->d_vol != nullptr;
   return ST_OK;
 }
+
+// The texture is (about to be) whole again.
+static void clear_gas_fault(st_context* ctx) {
+  if (!ctx->gas_fault) return;
+  cudaStreamSynchronize(ctx->stream);  // steps that may still set it
+  *ctx->gas_fault = 0;
+}
+int context_gas_fault(st_context* ctx, int** dev) {
+  if (!ctx->gas_fault) {
+    void* h = nullptr;
+    if (cudaHostAlloc(&h, sizeof(int), cudaHostAllocMapped) != cudaSuccess) {
+      (void)cudaGetLastError();
+      return ST_ENOMEM;
+    }
+    ctx->gas_fault = static_cast<int*>(h);
+  }
+  clear_gas_fault(ctx);
+  return cudaHostGetDevicePointer((void**)dev, (void*)ctx->gas_fault, 0) == cudaSuccess ? ST_OK : ST_ECUDA;
+}
+bool context_gas_failed(st_context* ctx) { return ctx->gas_fault && *ctx->gas_fault != 0; }
 
 }  // namespace st
 
@@ -1362,7 +1391,7 @@ int layered_render(st_context* ctx, const st_camera* cam, const st_spacetime* st
   if (host_diag)
     ST_CUDA(cudaMemcpyAsync(host_diag, ctx->d_diag, npix * sizeof(st_ray_diag), cudaMemcpyDeviceToHost, s));
   ST_CUDA(cudaStreamSynchronize(s));
-  const int status = cnt[st::CNT_STATUS] ? (int)cnt[st::CNT_STATUS] : ST_OK;
+  const int status = launch_status(ctx, cnt);
   if (stats) {
     float ms = 0.f;
     if (cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1) != cudaSuccess) { (void)cudaGetLastError(); ms = 0.f; }
@@ -1497,6 +1526,7 @@ int st_context_set_volume(st_context* ctx, const st_volume* v) {
   if (!ctx->d_vol && cudaMalloc(&ctx->d_vol, n * sizeof(float)) != cudaSuccess) return ST_ENOMEM;
   if (cudaMemcpy(ctx->d_vol, v->density, n * sizeof(float), cudaMemcpyHostToDevice) != cudaSuccess)
     return ST_ECUDA;
+  st::clear_gas_fault(ctx);
   ctx->vol_bytes = n * sizeof(float);
   ctx->vol = *v;
   ctx->vol.density = nullptr;
@@ -1601,6 +1631,7 @@ void st_context_destroy(st_context* ctx) {
   if (ctx->ev_layer) cudaEventDestroy(ctx->ev_layer);
   if (ctx->lstream) cudaStreamDestroy(ctx->lstream);
   cudaFree(ctx->d_vol);
+  cudaFreeHost((void*)ctx->gas_fault);
   cudaFree(ctx->d_fb);
   cudaFree(ctx->d_rgb);
   cudaFree(ctx->d_diag);
@@ -1848,7 +1879,7 @@ int st_render_frames(st_context* ctx, int nframes, const st_camera* cams, const 
   ST_CUDA(cudaMemcpyAsync(out_rgb, ctx->d_rgb, 3 * npix * nframes * sizeof(float), cudaMemcpyDeviceToHost, s));
   ST_CUDA(cudaStreamSynchronize(s));
   const unsigned long long* cnt = ctx->h_cnt;
-  const int status = cnt[st::CNT_STATUS] ? (int)cnt[st::CNT_STATUS] : ST_OK;
+  const int status = launch_status(ctx, cnt);
   if (stats) {
     float ms = 0.f;
     // a failed query must not leave an error pending for the next launch check

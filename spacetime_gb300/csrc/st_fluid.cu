@@ -45,6 +45,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstdlib>
 #include <cstring>
 #include <vector>
 
@@ -147,6 +148,7 @@ struct Fields {
   float* t;                     // [2] simulation clock by parity
   unsigned* count;              // arrivals at the grid barrier, never reset
   int* status;                  // set when a barrier's wait ran out
+  int* fault;                   // and with it this word of the context, in host memory
   float* vol;                   // (nr, nphi, nz) density texture of the context
 };
 
@@ -157,16 +159,26 @@ constexpr int LOW = 8, TALL = 32;  // and along j: in the one launch, in launche
 // is then 64 cells along i: a thread owns one column of it, every eighth row.
 constexpr int MAX_SWEEPS = 15;
 constexpr int COLS = TI + 2 * (MAX_SWEEPS + 1), ROWS = THREADS / COLS;
-constexpr unsigned WAIT_LIMIT = 1u << 22;  // polls of a barrier, some seconds
+// Polls of a barrier, some seconds.  A constant of the kernel: as a parameter it
+// made the polling loop, and with it a step of 256 x 64 cells, 1.3 % slower.
+constexpr unsigned WAIT_LIMIT = 1u << 22;
 
 // Floats of shared memory of a pass: p twice.
 constexpr size_t tile_floats(int tj, int H) { return 2 * (size_t)(TI + 2 * H) * (tj + 2 * H); }
 static_assert(tile_floats(TALL, MAX_SWEEPS + 1) * sizeof(float) <= 48 * 1024, "no opt-in needed");
 
+// Tells the host, without a copy or a wait on its side: the next step of a solver
+// and the next render of the context look at this word.
+__device__ __forceinline__ void report_fault(const Fields& F) {
+  *static_cast<volatile int*>(F.fault) = 1;
+  __threadfence_system();
+}
+
 // All blocks of the (cooperative) launch; `target` counts their arrivals since
 // the counter's creation, modulo 2^32.  False, for the whole block, when the
 // wait ran out; the fields are then not to be used.  (A word a block that every
 // block polls instead of one counter took 30,000 cycles: 152 x 152 polls.)
+template <unsigned LIMIT>
 __device__ __forceinline__ bool grid_barrier(const Fields& F, unsigned target) {
   int out = 0;
   __syncthreads();
@@ -177,7 +189,12 @@ __device__ __forceinline__ bool grid_barrier(const Fields& F, unsigned target) {
     while (true) {
       asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(F.count) : "memory");
       if ((int)(v - target) >= 0) break;
-      if (++polls >= WAIT_LIMIT) { out = 1; atomicExch(F.status, 1); break; }
+      if (++polls >= LIMIT) {
+        out = 1;
+        atomicExch(F.status, 1);
+        report_fault(F);
+        break;
+      }
     }
   }
   return !__syncthreads_or(out);
@@ -361,14 +378,17 @@ __device__ __forceinline__ void extrude(const Fields& F, int idx, int i, float d
 // (even, or 0); `base` barrier arrivals before this launch.  Work of a phase is
 // dealt in whole warps, round the blocks, so that a few hundred warps of work
 // occupy every SM.
-template <int BLOCKS_SM>
+template <int BLOCKS_SM, unsigned LIMIT>
 __global__ void __launch_bounds__(THREADS, BLOCKS_SM)
     fluid_steps_kernel(Fields F, int parity, int nsteps, float dt, int sweeps, float amp, float drag, float relax,
                        unsigned base) {
   extern __shared__ float sm[];
   const unsigned nr = F.nr, n = nr * (unsigned)F.nphi;
   const unsigned warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (*static_cast<volatile int*>(F.status)) return;  // an earlier launch's wait ran out
+  if (*static_cast<volatile int*>(F.status)) {  // an earlier launch's wait ran out
+    if (blockIdx.x == 0 && threadIdx.x == 0) report_fault(F);
+    return;
+  }
   unsigned bars = base;
   // f(kind, idx, i, j) for `kinds` kinds of work on every cell, by blocks b of nb
   auto cells = [&](unsigned kinds, unsigned b, unsigned nb, auto f) {
@@ -389,7 +409,7 @@ __global__ void __launch_bounds__(THREADS, BLOCKS_SM)
   cells(1, blockIdx.x, gridDim.x, [&](int, int idx, int i, int j) {
     velocity_cell(F, idx, i, j, force_u(i, j, t), force_v(i, j, t), dt, amp, drag);
   });
-  if (!grid_barrier(F, bars += gridDim.x)) return;
+  if (!grid_barrier<LIMIT>(F, bars += gridDim.x)) return;
   for (int k = 0; k < nsteps; ++k) {
     const float tn = t + dt;
     const bool end = k + 1 == nsteps;
@@ -402,7 +422,7 @@ __global__ void __launch_bounds__(THREADS, BLOCKS_SM)
       for (int b = blockIdx.x; b < tiles; b += gridDim.x)
         pressure_tile<LOW>(F, b % gx, b / gx, first, sweeps > 0, src, m, left == 0, sm);
       if (left == 0) break;
-      if (!grid_barrier(F, bars += gridDim.x)) return;
+      if (!grid_barrier<LIMIT>(F, bars += gridDim.x)) return;
       src = 1 - src;
       first = false;
     }
@@ -412,7 +432,7 @@ __global__ void __launch_bounds__(THREADS, BLOCKS_SM)
         else if (kind == 1) F.fu[idx] = force_u(i, j, tn);
         else F.fv[idx] = force_v(i, j, tn);
       });
-    if (!grid_barrier(F, bars += gridDim.x)) return;
+    if (!grid_barrier<LIMIT>(F, bars += gridDim.x)) return;
     cells(end ? 1 : 2, blockIdx.x, gridDim.x, [&](int kind, int idx, int i, int j) {
       if (kind == 0) {
         const float dn =
@@ -423,7 +443,7 @@ __global__ void __launch_bounds__(THREADS, BLOCKS_SM)
                       amp, drag);
       }
     });
-    if (!end && !grid_barrier(F, bars += gridDim.x)) return;
+    if (!end && !grid_barrier<LIMIT>(F, bars += gridDim.x)) return;
     parity ^= 1;
     t = tn;
   }
@@ -482,6 +502,17 @@ namespace {
 constexpr int DENSE = 3;  // blocks an SM of the larger grids
 constexpr int LAUNCH_STEPS = 1024;  // steps of one launch, some milliseconds
 
+// The one-launch kernel for `blocks` blocks.  SPACETIME_GB300_FLUID_WAIT=1 in the
+// environment takes the kernels whose barriers give up after one poll, so a test can
+// make a wait run out (the blocks then leave the launch one by one, the fields are
+// not to be used, and the solver and the context report it).
+const void* steps_kernel(bool dense) {
+  const char* e = std::getenv("SPACETIME_GB300_FLUID_WAIT");
+  if (e && std::strcmp(e, "1") == 0)
+    return dense ? (const void*)fluid_steps_kernel<DENSE, 1> : (const void*)fluid_steps_kernel<1, 1>;
+  return dense ? (const void*)fluid_steps_kernel<DENSE, WAIT_LIMIT> : (const void*)fluid_steps_kernel<1, WAIT_LIMIT>;
+}
+
 // `nsteps` (<= LAUNCH_STEPS) steps from the current parity on stream s.
 int launch_steps(st_fluid* f, float* vol, int nsteps, float dt, int jacobi, cudaStream_t s) {
   Fields F = f->F;
@@ -523,8 +554,7 @@ int launch_steps(st_fluid* f, float* vol, int nsteps, float dt, int jacobi, cuda
   }
   const unsigned blocks = (unsigned)std::min(
       most, std::max(std::min<size_t>(f->num_sms, (cells + 63) / 64), tiles + tiles / 2));
-  const void* kernel =
-      blocks > (unsigned)f->num_sms ? (const void*)fluid_steps_kernel<DENSE> : (const void*)fluid_steps_kernel<1>;
+  const void* kernel = steps_kernel(blocks > (unsigned)f->num_sms);
   const size_t smem = tile_floats(LOW, widest) * sizeof(float);
   int parity = f->parity;
   float amp = (float)f->forcing, drag = (float)f->drag, relax = (float)f->relax;
@@ -601,6 +631,9 @@ int st_fluid_create(st_fluid** out, st_context* ctx, const st_disc* disc, const 
     }
     shear[i - 1] = (float)(std::sqrt(M / (s * s * s)) * nphi / (2.0 * 3.141592653589793));
   }
+  int* fault = nullptr;
+  const int frc = st::context_gas_fault(ctx, &fault);
+  if (frc != ST_OK) return frc;
   st_fluid* f = new st_fluid;
   f->ctx = ctx;
   f->device = cv.device;
@@ -631,6 +664,7 @@ int st_fluid_create(st_fluid** out, st_context* ctx, const st_disc* disc, const 
   F.count = reinterpret_cast<unsigned*>(F.t + 2);
   F.status = reinterpret_cast<int*>(F.t + 3);
   F.base = base_d; F.env = env_d; F.shear = shear_d;
+  F.fault = fault;
   bool ok = cudaMemsetAsync(b, 0, total * sizeof(float), f->stream) == cudaSuccess;
   ok = ok && cudaMemcpyAsync(F.dens[0], dens0.data(), n * sizeof(float), cudaMemcpyHostToDevice, f->stream) ==
                  cudaSuccess;
@@ -659,6 +693,7 @@ int st_fluid_step(st_fluid* f, double dt, int jacobi, int nsteps, int, float* ms
   if (st::context_volume(f->ctx, &cv) != ST_OK || !cv.on || cv.meta.nr != f->nr || cv.meta.nphi != f->nphi ||
       cv.meta.nz != f->nz)
     return ST_ESTATE;
+  if (st::context_gas_failed(f->ctx)) return ST_ECUDA;
   // the steps run on the context's stream, so the next render sees the field
   cudaStream_t s = cv.stream;
   cudaEvent_t e0 = nullptr, e1 = nullptr;

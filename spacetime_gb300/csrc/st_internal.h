@@ -22,6 +22,11 @@ struct CtxVolume {
   bool on;
 };
 int context_volume(st_context* ctx, CtxVolume* out);
+// The context's word, in host memory that kernels can write, by which a fluid
+// solver that gave up says that the density texture is not to be used: its device
+// address (cleared: a new solver), and whether it is set.
+int context_gas_fault(st_context* ctx, int** dev);
+bool context_gas_failed(st_context* ctx);
 
 // Counters written by the trace kernels (one slot each, 64-bit).
 enum { CNT_STEPS = 0, CNT_FP64 = 1, CNT_GAS = 2, CNT_RAYS = 3, CNT_SURR = 4, CNT_QUEUE = 5,
