@@ -583,11 +583,11 @@ ST_DF dd fma1(dd a, dd b, dd x) { return add(x, mul(a, b)); }
 // below the pair terms fit a float.
 
 // e^x, x <= 80: x = n ln 2 + r, e^(r/16) - 1 by Taylor's series, and four times
-// (1 + s)^2 - 1 = 2 s + s^2.  Below -87, where 2^n would leave a float's normal
-// exponents, it is e^-87 (the argument may be -infinity: an optical depth is as large
+// (1 + s)^2 - 1 = 2 s + s^2.  Below -87.3, where 2^n would leave a float's normal
+// exponents, it is e^-87.3 (the argument may be -infinity: an optical depth is as large
 // as the user's opacity, spacing and density make it).
 ST_DF df2 exp_(df2 x) {
-  if (x.hi < -87.f) x = q(-87.f);
+  if (x.hi < -87.3f) x = q(-87.3f);
   const float n = rintf(fmul(x.hi, 1.44269504f));
   // ln 2 in three floats
   const float p = fmul(n, 0.693147182f), pe = ffma(n, 0.693147182f, -p);

@@ -4,7 +4,7 @@ user chooses opacity, spacing and density, so -x has no bound.
 
 Tolerance: 2^-36 relative (as tests/test_df_math.py asks of the normal range)
 down to -80; below, where the result's low half leaves a float's normal
-exponents, one float rounding, 2^-23, or, below -87, e^-87.  A sample's emission
+exponents, one float rounding, 2^-23, and e^-87, where it ends.  A sample's emission
 1 - e^x and the transmittance behind it stay in [0, 1].
 """
 import math
