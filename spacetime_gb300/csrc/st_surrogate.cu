@@ -1655,6 +1655,7 @@ struct st_surrogate {
   int* fCount = nullptr;      // per warp: their number
   int* fOff = nullptr;        // per warp: offset in the list
   long long frows = 0;
+  int rows = 0;  // capacity of a call's own rows (X, T)
   int cap = 0;  // rows of the work buffers
   float* X = nullptr;
   float* Z[4] = {nullptr, nullptr, nullptr, nullptr};
@@ -1678,24 +1679,36 @@ using namespace st::sur;
     if ((call) != cudaSuccess) return ST_ECUDA; \
   } while (0)
 
+// A call's own inputs and targets.
+int ensure_rows(st_surrogate* s, int rows) {
+  if (rows <= s->rows) return ST_OK;
+  cudaFree(s->X); cudaFree(s->T);
+  s->X = s->T = nullptr;
+  s->rows = 0;
+  if (cudaMalloc(&s->X, (size_t)rows * NIN * 4) != cudaSuccess || cudaMalloc(&s->T, (size_t)rows * NT * 4) != cudaSuccess)
+    return ST_ENOMEM;
+  s->rows = rows;
+  return ST_OK;
+}
+
+// What the layer-by-layer kernels keep besides.
 int ensure_work(st_surrogate* s, int rows) {
   if (rows <= s->cap) return ST_OK;
-  cudaFree(s->X);
   for (int l = 0; l < 4; ++l) { cudaFree(s->Z[l]); cudaFree(s->H[l]); }
-  cudaFree(s->dZa); cudaFree(s->dZb); cudaFree(s->out); cudaFree(s->dout); cudaFree(s->T);
+  cudaFree(s->dZa); cudaFree(s->dZb); cudaFree(s->out); cudaFree(s->dout);
   cudaFree(s->part);
-  s->part = nullptr;
+  for (int l = 0; l < 4; ++l) { s->Z[l] = nullptr; s->H[l] = nullptr; }
+  s->dZa = s->dZb = nullptr;
+  s->out = s->dout = s->part = nullptr;
   s->cap = 0;
   const size_t R = rows;
-  if (cudaMalloc(&s->X, R * NIN * 4) != cudaSuccess) return ST_ENOMEM;
   for (int l = 0; l < 4; ++l) {
     if (cudaMalloc(&s->Z[l], R * NH * 4) != cudaSuccess) return ST_ENOMEM;
     if (cudaMalloc(&s->H[l], R * NH * 2) != cudaSuccess) return ST_ENOMEM;
   }
   if (cudaMalloc(&s->dZa, R * NH * 2) != cudaSuccess || cudaMalloc(&s->dZb, R * NH * 2) != cudaSuccess)
     return ST_ENOMEM;
-  if (cudaMalloc(&s->out, R * NOUT * 4) != cudaSuccess || cudaMalloc(&s->dout, R * NOUT * 4) != cudaSuccess ||
-      cudaMalloc(&s->T, R * NT * 4) != cudaSuccess)
+  if (cudaMalloc(&s->out, R * NOUT * 4) != cudaSuccess || cudaMalloc(&s->dout, R * NOUT * 4) != cudaSuccess)
     return ST_ENOMEM;
   if (cudaMalloc(&s->part, (R / RED_ROWS + 1) * (size_t)L0_PART * 4) != cudaSuccess) return ST_ENOMEM;
   s->cap = rows;
@@ -2060,7 +2073,8 @@ int st_surrogate_forward(st_surrogate* s, const float* X, int n, float* out) {
   if (!s || !X || !out || n <= 0) return ST_EINVAL;
   if (cudaSetDevice(s->device) != cudaSuccess) return ST_ECUDA;
   const int B = pad128(n);
-  int rc = ensure_work(s, B);
+  int rc = ensure_rows(s, B);
+  if (rc == ST_OK) rc = ensure_work(s, B);
   if (rc != ST_OK) return rc;
   SC(cudaMemsetAsync(s->X, 0, (size_t)B * NIN * 4, s->stream));
   SC(cudaMemcpyAsync(s->X, X, (size_t)n * NIN * 4, cudaMemcpyHostToDevice, s->stream));
@@ -2102,7 +2116,9 @@ int st_surrogate_loss_grad(st_surrogate* s, const float* X, const float* T, int 
   if (!s || !X || !T || n <= 0) return ST_EINVAL;
   if (cudaSetDevice(s->device) != cudaSuccess) return ST_ECUDA;
   const int B = pad128(n);
-  int rc = ensure_work(s, B);
+  const bool tc5 = train_on_tcgen05();
+  int rc = ensure_rows(s, B);
+  if (rc == ST_OK) rc = tc5 ? ensure_train(s, B / (int)TC_ROWS) : ensure_work(s, B);
   if (rc != ST_OK) return rc;
   cudaStream_t st = s->stream;
   SC(cudaMemsetAsync(s->X, 0, (size_t)B * NIN * 4, st));
@@ -2110,8 +2126,7 @@ int st_surrogate_loss_grad(st_surrogate* s, const float* X, const float* T, int 
   SC(cudaMemcpyAsync(s->X, X, (size_t)n * NIN * 4, cudaMemcpyHostToDevice, st));
   SC(cudaMemcpyAsync(s->T, T, (size_t)n * NT * 4, cudaMemcpyHostToDevice, st));
   SC(cudaMemsetAsync(s->loss, 0, 16 * 4, st));
-  if (train_on_tcgen05()) {
-    if ((rc = ensure_train(s, B / (int)TC_ROWS)) != ST_OK) return rc;
+  if (tc5) {
     if ((rc = train_pass(s, s->X, s->T, B, n, s->loss, s->G, AdamParams{})) != ST_OK) return rc;
   } else {
     if ((rc = forward(s, s->X, B, true, s->stream)) != ST_OK) return rc;
