@@ -1870,7 +1870,8 @@ int ensure_train(st_surrogate* s, int ntiles) {
       cudaMalloc(&s->tpart, 4 * nt * TR_ROW * sizeof(float)) != cudaSuccess ||
       cudaMalloc(&s->tpw, (size_t)train_splits(ntiles) * 3 * NH * NH * sizeof(float)) != cudaSuccess)
     return ST_ENOMEM;
-  SC(cudaFuncSetAttribute(train_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TR_SMEM));
+  for (auto* k : {train_tile_kernel<false>, train_tile_kernel<true>})
+    SC(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TR_SMEM));
   SC(cudaFuncSetAttribute(train_dw_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DW_SMEM));
   // all three kernels of a step on one split of L1, so no SM changes it between them
   SC(cudaFuncSetAttribute(train_update_kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
@@ -1896,6 +1897,20 @@ cudaError_t launch_dependent(void (*kernel)(P...), dim3 grid, int threads, size_
   return cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...);
 }
 
+// Wait bound and first-copy switch of sur_mlp_tc_kernel and train_tile_kernel.  The environment
+// variable SPACETIME_GB300_TC_WAIT_OUT=1 makes every CTA's first wait run out
+// (its first copies are never issued, short wait bound), so all tiles fail:
+// the failure path under test.
+struct TcWait {
+  uint32_t limit;
+  int issue_first;
+};
+TcWait tc_wait_mode() {
+  const char* e = std::getenv("SPACETIME_GB300_TC_WAIT_OUT");
+  if (e && std::strcmp(e, "1") == 0) return TcWait{1024u, 0};
+  return TcWait{TC_WAIT_LIMIT, 1};
+}
+
 // Loss sums (added to loss[4]) and gradient of B padded rows, n of which count,
 // into G or, where G is null, an AdamW step.
 int train_pass(st_surrogate* s, const float* X, const float* T, int B, int n, float* loss, float* G,
@@ -1904,7 +1919,8 @@ int train_pass(st_surrogate* s, const float* X, const float* T, int B, int n, fl
   // (rounded up to whole blocks of 64 rows, the last of 64 shares may be empty)
   const int per = (2 * nt + train_splits(nt) - 1) / train_splits(nt), splits = (2 * nt + per - 1) / per;
   const TrainParams tp{s->P, s->WF, s->WT, X, T, n, nt, 1.0f / n, s->tH, s->tD, s->tZ, s->tpart, loss, s->d_status};
-  SC(launch_dependent(train_tile_kernel, grid, TR_THREADS, TR_SMEM, s->stream, tp));
+  const bool run_out = !tc_wait_mode().issue_first;
+  SC(launch_dependent(run_out ? train_tile_kernel<true> : train_tile_kernel<false>, grid, TR_THREADS, TR_SMEM, s->stream, tp));
   SC(launch_dependent(train_dw_kernel, dim3(splits, 2, 3), 256, DW_SMEM, s->stream, s->tH, s->tD, nt, s->tpw,
                       s->d_status));
   SC(launch_dependent(train_update_kernel, UPD_HIDDEN + UPD_EDGE, 256, 0, s->stream, s->tpw, splits, s->tpart, 4 * nt,
@@ -1924,20 +1940,6 @@ int gemm_status(st_surrogate* s) {
     return ST_ECUDA;
   }
   return ST_OK;
-}
-
-// Wait bound and first-copy switch of sur_mlp_tc_kernel.  The environment
-// variable SPACETIME_GB300_TC_WAIT_OUT=1 makes every CTA's first wait run out
-// (its first copies are never issued, short wait bound), so all tiles fail:
-// the failure path under test.
-struct TcWait {
-  uint32_t limit;
-  int issue_first;
-};
-TcWait tc_wait_mode() {
-  const char* e = std::getenv("SPACETIME_GB300_TC_WAIT_OUT");
-  if (e && std::strcmp(e, "1") == 0) return TcWait{1024u, 0};
-  return TcWait{TC_WAIT_LIMIT, 1};
 }
 
 // Frame-pass buffers for `rows` network rows (a multiple of 128, one tile of

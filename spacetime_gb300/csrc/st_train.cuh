@@ -123,6 +123,9 @@ __device__ __forceinline__ void row8(const float* r, float* v) {
   v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
 }
 
+// RUN_OUT: the first copy is left out, so that each CTA's first wait runs out (the
+// failure path under test).
+template <bool RUN_OUT>
 __global__ void __launch_bounds__(TR_THREADS, 1) train_tile_kernel(const TrainParams tp) {
   extern __shared__ unsigned char tr_raw[];
   unsigned char* base = reinterpret_cast<unsigned char*>(
@@ -158,7 +161,7 @@ __global__ void __launch_bounds__(TR_THREADS, 1) train_tile_kernel(const TrainPa
   uint32_t pw = 0, pm = 0;
   bool w_out = false, m_out = false;  // thread 0: a copy or a product is in flight
   wait_for_previous();
-  if (tid == 0) {
+  if (tid == 0 && !RUN_OUT) {
     load_w(0);
     w_out = true;
   }
@@ -259,7 +262,7 @@ __global__ void __launch_bounds__(TR_THREADS, 1) train_tile_kernel(const TrainPa
       if (m == 5 && t + (int)gridDim.x >= tp.ntiles) let_next_start();
       if (tid == 0) {
         tc::fence_after_sync();
-        if (!tc::mbar_wait(&S.bar_w, pw, TC_WAIT_LIMIT)) {
+        if (!tc::mbar_wait(&S.bar_w, pw, RUN_OUT ? 1024u : TC_WAIT_LIMIT)) {
           S.fail = 1;
         } else {
           w_out = false;
