@@ -11,9 +11,10 @@
 // which do not depend on what lies in front) in parallel, and one of them blends
 // each ray's samples in order.  A ray found opaque ends with the state of that
 // sample's step, from the buffer; the steps that the integrator took beyond are
-// dropped.  The arithmetic of steps and samples is the pixel kernel's, to the bit.
-// 64x36 Kerr gas: 1.97 -> 1.01 ms; with 8 steps a batch 1.16, with seven shading
-// warps 1.10.
+// dropped.  The arithmetic of steps and samples is the pixel kernel's: 120 random
+// gas frames had the same bits as that kernel gave them.
+// 64x36 Kerr gas: 2.05 -> 1.07 ms (an earlier build 1.01; there 1.16 with 8 steps a
+// batch, 1.10 with seven shading warps).
 #pragma once
 
 #include "st_kernels.cuh"
@@ -230,13 +231,22 @@ __global__ void __launch_bounds__(32 * (1 + SPLIT_SHADERS)) trace_split_kernel(c
 }
 
 // The rule: whole FP32 gas frames of the pixel schedule with so few rays in flight
-// that a step's latency and not its instructions are the frame's time.  The
-// line (ms, Kerr / Schwarzschild, pixel kernel -> this): 320x180 2.60 / 1.99 -> 2.35 / 1.74,
-// 400x225 3.37 / 2.12 -> 3.25 / 2.59, 480x270 3.68 / 2.40 -> about 4.5 / 3.1.
-constexpr long long SPLIT_RAYS = 65536;
+// that a step's latency and not its instructions are the frame's time.  Where the
+// line lies depends on how many of a ray's steps have samples, so it was set by
+// random scenes (spins, radii from 1.3 to 90 M, slabs, opacities to 3,000, strides to
+// 16, steps to 0.2; 10 to 49 a size).  Times against the pixel kernel's, geometric
+// mean, and how many frames of 0.1 ms or more were slower:
+//   64x36 0.79, none; 128x72 0.65, none; 160x90 0.69, none; 200x113 (22,600 rays)
+//   0.86, none, shorter ones by up to 28 us; 240x135 (32,400) 0.84, 3, by up to 117 us;
+//   280x158 1.01, 3; 300x169 1.14, 6; 256x256 1.10, 10, by up to 0.5 ms.
+// Near the horizon of a fast hole a step's samples run to hundreds, most of them
+// below the slab's inner edge, and all shading warps walk past all of them: 120x90
+// from 55 M with samples every step or two, spin 0.95 0.71 to 0.80 of the pixel
+// kernel's time, 0.99 0.94 to 1.24, 0.998 1.15 to 1.34 (every fourth step: 0.96).
+constexpr long long SPLIT_RAYS = 24576;
 inline bool split_takes(const Variant& v, const TraceParams& p) {
   return v.vol && v.sem == ST_SEM_DRAFT && v.sched == ST_SCHED_PIXEL && p.order == 4 && p.nb == 0 && !p.layer &&
-         !p.pix_list && !p.frames && p.box_cols <= 0 &&
+         !p.pix_list && !p.frames && p.box_cols <= 0 && (p.a <= 0.96 * p.M || p.ds_gas >= 3.5 * p.dt) &&
          (long long)p.width * p.height * (p.beside > 1 ? p.beside : 1) <= SPLIT_RAYS;
 }
 inline cudaError_t launch_split(const Variant& v, const TraceParams& p, cudaStream_t s) {
