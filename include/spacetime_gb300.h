@@ -92,7 +92,10 @@ enum {
   ST_PREC_FP64 = 0,          /* double accuracy: everything in double, or (RK4
                                 frames of the pixel schedule) slopes in pairs
                                 of floats and the state in three, whose error
-                                against the exact RK4 sequence is smaller */
+                                against the exact RK4 sequence is smaller.
+                                ST_SCHED_PERSISTENT keeps everything in double;
+                                camera tracks use it unless told otherwise, and
+                                are several times as fast on ST_SCHED_PIXEL */
   ST_PREC_FP32_GUARDED = 1,  /* FP32 RK4 with a compensated (float-float) state;
                                 steps inside r_guard, of rays in the critical
                                 band, and the null-constraint renormalisation

@@ -487,7 +487,10 @@ def step_sim(sim: DiscFluidSim, ctx: Context | None = None, *, dt: float = 0.05,
 
 def render_frames(ctx: Context, cams, bh, *, width: int, height: int, dt: float = 0.02, precision="fp32g",
                   **kw) -> np.ndarray:
-    """A camera track rendered in one persistent launch (DRAFT semantics)."""
+    """A camera track rendered in one persistent launch (DRAFT semantics).  In
+    FP64 the persistent kernels are all double: a track on pixel tiles
+    (`Context.render_frames_raw` with `schedule=ST_SCHED_PIXEL`) integrates in float
+    pairs and is several times as fast."""
     p = ctx.params(_abi.ST_SEM_DRAFT, width=width, height=height, samples=1, dt=dt,
                    precision=_prec(precision), pixel_jitter=0, schedule=_abi.ST_SCHED_PERSISTENT, **kw)
     return ctx.render_frames_raw(cams, bh, p).image

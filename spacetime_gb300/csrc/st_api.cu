@@ -421,11 +421,12 @@ double norm3(const double* v) { return std::sqrt(v[0] * v[0] + v[1] * v[1] + v[2
 
 // FP32_GUARDED on the pixel schedule (RK4, no depth buckets), with the
 // environment variable SPACETIME_GB300_GUARD_DEFER=1: space for every ray of
-// one launch to be saved before its first FP64 guard step, so the guard steps
-// run in full warps of a resume kernel.  Off by default: on the 1080p config-1
-// frame the split measured slower than the guard steps inline (103.2 vs
-// 94.5 ms), because the resumed rays' FP64 work no longer overlaps the
-// other warps' FP32 work and their FP64 segments end at different steps.
+// one launch to be saved before its first guard step, so the guard steps
+// run in full warps of a resume kernel.  Off by default: the split is slower than
+// the guard steps inline (Kerr gas, guards inside 3 M: 1080p 55.5 against 46.3 ms,
+// 480x270 11.8 against 9.9; thin disc 41.2 against 33.7 and 9.2 against 6.7),
+// because the resumed rays' guard steps no longer overlap the other warps' work
+// and their guarded stretches end at different steps.
 int setup_defer(st_context* ctx, TraceParams* p, const st::Variant& v, size_t nrays) {
   p->defer_state = nullptr;
   p->defer_count = nullptr;
@@ -757,9 +758,9 @@ long long queue_budget(long long computed) {
 
 // Centre-first dispatch order of a full-frame pixel launch.  A block's cost is
 // its slowest ray, and the slowest rays sit near the hole: on the 1080p
-// config-1 frame with FP64 guard steps the longest blocks run 70-84 ms, and in
-// raster order they start 20-27 ms into a frame whose blocks average 1.6 ms,
-// so the frame ends on them.  Tiles are sorted by Chebyshev distance, in
+// config-1 frame with guard steps in double (as they were when this was measured)
+// the longest blocks ran 70-84 ms, and in raster order they started 20-27 ms into a
+// frame whose blocks averaged 1.6 ms, so the frame ended on them.  Tiles are sorted by Chebyshev distance, in
 // tiles, from the tile the hole projects into (pinhole projection of the
 // direction to the origin on the camera's axes; the frame centre when the hole
 // is behind the camera or the lens is a fisheye), nearest first: a counting

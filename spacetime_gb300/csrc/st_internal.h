@@ -130,10 +130,10 @@ struct TraceParams {
   // pixel schedule over a compacted list (surrogate fallback rays)
   const int* pix_list;       // optional pixel indices (device)
   const int* n_list;         // their count (device)
-  // FP32_GUARDED pixel schedule: rays stop before their first FP64 guard step
+  // FP32_GUARDED pixel schedule: rays stop before their first guard step
   // and are saved here (defer_cap states of the trace unit's ray-state size,
   // in the order their warps reached it); a resume kernel over the saved
-  // rays runs the FP64 steps in full warps.  Null: guard steps inline.
+  // rays runs the guard steps in full warps.  Null: guard steps inline.
   void* defer_state;
   unsigned int* defer_count;
   int defer_cap;

@@ -127,8 +127,8 @@ __global__ void __launch_bounds__(128, ORD != 4 ? ST_MINB_ADAPTIVE : KERR && !VO
   flush_counters(p, steps, f64, gas, rays);
 }
 
-// FP32_GUARDED: the rays the pixel kernel saved before their first FP64 step,
-// one thread each, so the FP64 steps they start with run in full warps; each
+// FP32_GUARDED: the rays the pixel kernel saved before their first guard step,
+// one thread each, so the guard steps they start with run in full warps; each
 // continues to its end with the guard steps inline.
 template <int KERR, int VOL, int SEM>
 __global__ void __launch_bounds__(128, ST_MINB) trace_resume_kernel(const __grid_constant__ TraceParams p) {
@@ -276,7 +276,7 @@ cudaError_t launch_variant(const TraceParams& p, int sched, int bx, int by, int 
     if constexpr (PREC == ST_PREC_FP32_GUARDED) {
       if (p.defer_state && p.defer_count && p.defer_cap > 0) {
         // guard steps gathered into full warps: stop each ray before its first
-        // FP64 step, then resume the saved rays one per thread
+        // guard step, then resume the saved rays one per thread
         cudaError_t e = cudaMemsetAsync(p.defer_count, 0, sizeof(unsigned int), s);
         if (e != cudaSuccess) return e;
         trace_pixel_kernel<PREC, KERR, VOL, SEM, 4, 0, 1><<<grid, block, 0, s>>>(p);

@@ -22,7 +22,8 @@
 // accumulation (st_mlp.cuh); the 6->256 and 256->6 layers, the loss and AdamW
 // run in FP32.  Master weights and optimiser state are FP32.
 //
-// Training labels come from the FP64 integrator on the GPU (label_pairs_kernel):
+// Training labels come from a double-accuracy integrator on the GPU, in float pairs
+// (label_pairs_kernel; double outside its range of steps):
 // Sobol-sampled inputs, the kernel's step rule and kill tests
 // (src/metal.jl:1201-1572) with the spin per sample, exit direction on the
 // escape radius 2 max(|pos|, 15M) (src/metal.jl:2058-2059).
@@ -2165,7 +2166,8 @@ int st_surrogate_generate(st_surrogate* s, long long n, long long offset, double
     // Warps per SM: two per scheduler fill the FP32 pipe; more only make every
     // step, and so the longest ray, slower (131,072 labels: 24.3 ms with 8 an SM,
     // 30.7 with 12; 2^20: 127 ms with either), and a small set ends with its
-    // longest ray (65,536 labels: 16.3 ms with 4 an SM, 21.3 with 8).
+    // longest ray (65,536 labels: 16.3 ms with 4 an SM, 21.3 with 8).  The line is at
+    // the smaller of the two sizes measured: a set of one more takes 17.0 ms for 14.5.
     int nsm = 0;
     SC(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, s->device));
     const long long warps = std::min((n + 31) / 32, (long long)nsm * (n <= 65536 ? 4 : LABEL_WARPS));

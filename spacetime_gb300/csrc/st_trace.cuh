@@ -8,7 +8,8 @@
 //   SEM = ST_SEM_RENDER  render / _trace_color (src/raytrace.jl:225-428,
 //                        src/callbacks.jl:7-105, src/accretion_disc.jl:19-49)
 // Precision:
-//   ST_PREC_FP64          all double
+//   ST_PREC_FP64          all double (the kernels of st_trace_pairs.cu, which take
+//                         most of these frames, are apart)
 //   ST_PREC_FP32          all float (the reference kernel's arithmetic)
 //   ST_PREC_FP32_GUARDED  float RHS, float-float (TwoSum) state, float-pair
 //                         steps for guarded rays/regions, and the same for the
@@ -560,7 +561,7 @@ __device__ __forceinline__ bool final_at_launch(const TraceParams& p, int flags)
 // Internal ray flag of the layer pass: the fan proves the ray misses the gate.
 constexpr int ST_RAY_LAYER_CULLED = 1 << 20;
 // Internal ray flag of the guarded schedule: the ray stopped before its first
-// FP64 guard step, its state saved for the resume kernel.
+// guard step, its state saved for the resume kernel.
 constexpr int ST_RAY_DEFER = 1 << 21;
 constexpr int ST_RAY_INTERNAL = ST_RAY_LAYER_CULLED | ST_RAY_DEFER;
 
@@ -1208,10 +1209,10 @@ __device__ __forceinline__ void null_renorm(float* y, float* lo, float ptf, cons
 // One integration step for the variant; returns true when the ray is done.
 // Mirrors the step loop of src/metal.jl:1201-1572 (DRAFT) and the callback
 // structure of src/raytrace.jl:339-373 (RENDER).  DEFER (FP32_GUARDED): a
-// step that would run in FP64 is not taken; the ray returns flagged
+// step that would be a guard step is not taken; the ray returns flagged
 // ST_RAY_DEFER with its state as it entered the call (the only field the
 // call has written, r_prev, is rewritten to the same value when the step is
-// taken again), so the resume kernel can take it in a dense FP64 warp.
+// taken again), so the resume kernel can take it in a dense warp of guard steps.
 // The gas along a step is `gas`'s to march (VOL; true ends the ray).
 template <int PREC, int KERR, int VOL, int SEM, int ORD = 4, int DEPTH = 0, int DEFER = 0, class Gas = MarchGas>
 __device__ __forceinline__ bool step_ray(const TraceParams& p, RayState<typename RealOf<PREC>::T>& st,
