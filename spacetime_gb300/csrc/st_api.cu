@@ -760,11 +760,11 @@ long long queue_budget(long long computed) {
 // its slowest ray, and the slowest rays sit near the hole: on the 1080p
 // config-1 frame with guard steps in double (as they were when this was measured)
 // the longest blocks ran 70-84 ms, and in raster order they started 20-27 ms into a
-// frame whose blocks averaged 1.6 ms, so the frame ended on them.  Tiles are sorted by Chebyshev distance, in
-// tiles, from the tile the hole projects into (pinhole projection of the
-// direction to the origin on the camera's axes; the frame centre when the hole
-// is behind the camera or the lens is a fisheye), nearest first: a counting
-// sort, O(tiles).  The order only moves when the grid or that tile changes.
+// frame whose blocks averaged 1.6 ms, so the frame ended on them.  Tiles are sorted
+// by Chebyshev distance, in tiles or in pixels, from the tile the hole projects into
+// (pinhole projection of the direction to the origin on the camera's axes; the frame
+// centre when the hole is behind the camera or the lens is a fisheye), nearest first:
+// a counting sort, O(tiles).  The order only moves when the grid or that tile changes.
 //
 // `pixels`: the distance in pixels, the sides of a 16x8 tile counted as they are.  The
 // rays that wind longest lie on a circle around the hole, and counted in tiles its
@@ -773,7 +773,8 @@ long long queue_budget(long long computed) {
 // default guards, medians of passes 21.1 to 27.0 ms, now 19.1 to 20.2; 480x270 Kerr
 // without matter 11.7 -> 9.3; FP64 320x180 disc 9.5 -> 8.9 and gas 18.6 -> 17.6.  The
 // plain float frames keep the distance in tiles, which suits them as well or better
-// (1080p gas 34.86 against 35.06 ms, two layered frames 3.68 against 3.73).
+// (1080p gas 34.86 against 35.06 ms, two layered frames 3.68 against 3.73), as do the
+// queue and the layer pass, whose order was not measured by pixels.
 bool round_order(const st::Variant& v) { return v.prec != ST_PREC_FP32; }
 int ensure_tile_order(st_context* ctx, const st_camera* cam, int width, int height, int bx, int by, bool pixels,
                       cudaStream_t s, const int** out) {

@@ -1150,7 +1150,9 @@ __device__ __forceinline__ R tsit5_adaptive(const R* s0, R pt, R M, R a, R r, R 
 // same sums went through fewer but slower instructions: the busiest scheduler of
 // a 640x360 Schwarzschild disc frame issued 0.65 a cycle, plain 0.81, and the
 // Kerr step spilled its loop's registers (28 to 436 bytes; plain none).  Guards
-// at their defaults, ms, in an earlier double-float step / packed / plain:
+// at their defaults, ms, in an earlier double-float step / packed / plain (all with
+// tiles dispatched by their distance in tiles; by pixels, ensure_tile_order in
+// st_api.cu, plain takes 5.2 and 9.3 for the first and third 480x270 here):
 // Schwarzschild disc 480x270 6.5 / 7.5 / 6.5, 640x360 7.3 / 8.6 / 7.4, 1080p 22.9 /
 // 22.6 / 21.6; Kerr without matter 480x270 16.6 / 15.0 / 11.7, 1080p 41.0 / 39.1 / 37.4;
 // Kerr gas 480x270 18.8 / 17.4 / 15.1, 1080p 64.0 / 59.0 / 53.3 (134 in double).

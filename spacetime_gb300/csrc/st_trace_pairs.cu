@@ -10,7 +10,7 @@
 // (tests/test_df_math.py).  Bound by the FP32 issue and pipe (58-67 % of the FMA
 // pipe) and, on small frames, by the longest ray's own chain of steps.  Measured
 // per frame, all-double before: 320x180 Schwarzschild disc by the CPU renderer's
-// rules 53.8 -> 9.5 ms, 320x180 Kerr gas 130 -> 18.0 ms.
+// rules 53.8 -> 8.9 ms, 320x180 Kerr gas 130 -> 17.6 ms.
 #include "st_kernels.cuh"
 
 namespace st {
